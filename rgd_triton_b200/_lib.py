@@ -110,6 +110,24 @@ def load() -> C.CDLL:
     return lib
 
 
+_host = None
+
+
+def host():
+    """The native host path (the extension module ``_host``), bound to the loaded library.  Raises if it
+    has not been built: on a GPU there is no slower path to fall back to silently."""
+    global _host
+    if _host is None:
+        try:
+            from . import _host as module
+        except ImportError as e:
+            raise RuntimeError("rgd_triton_b200/_host.so is missing or does not load: build it with "
+                               f"`python -m rgd_triton_b200.build` ({e})") from e
+        module.bind(load()._handle)
+        _host = module
+    return _host
+
+
 def status_string(code: int) -> str:
     return load().rgd_status_string(int(code)).decode()
 

@@ -4,7 +4,9 @@
 
 Every ``csrc/*.cu`` is compiled to an object file under ``csrc/build/`` (in
 parallel, skipped when the object is newer than the source and the headers) and
-linked into ``rgd_triton_b200/librgd_b200.so``.  No GPU is needed to build.
+linked into ``rgd_triton_b200/librgd_b200.so``; ``csrc/host/torch_host.cpp``, the
+native host path on top of the C ABI, becomes the extension module
+``rgd_triton_b200/_host.so``.  No GPU is needed to build.
 """
 from __future__ import annotations
 
@@ -20,6 +22,8 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 OBJ = CSRC / "build"
 LIB = PKG / "librgd_b200.so"
+HOST_SRC = CSRC / "host" / "torch_host.cpp"
+HOST_LIB = PKG / "_host.so"
 INCLUDE = PKG.parent / "include"
 
 NVCC_FLAGS = [
@@ -60,6 +64,28 @@ def _compile(src: Path, force: bool, verbose: bool, ptxas_v: bool) -> tuple[Path
     return obj, res.stderr
 
 
+def _build_host(force: bool, verbose: bool) -> None:
+    """The extension module (plain C++ against torch's headers; it finds librgd_b200.so at run time)."""
+    newest_dep = max(p.stat().st_mtime for p in (HOST_SRC, INCLUDE / "rgd_b200.h", Path(__file__)))
+    if not force and HOST_LIB.exists() and HOST_LIB.stat().st_mtime >= newest_dep:
+        return
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+    torch_lib = Path(torch.__file__).resolve().parent / "lib"
+    cuda_inc = Path(_nvcc()).resolve().parent.parent / "include"
+    incs = [*cpp_extension.include_paths(), sysconfig.get_paths()["include"], str(cuda_inc)]
+    cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *[f"-I{i}" for i in incs], str(HOST_SRC), "-o", str(HOST_LIB), f"-L{torch_lib}",
+           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python", "-ldl"]
+    if verbose:
+        print(" ".join(cmd), flush=True)
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"g++ failed for {HOST_SRC.name}:\n{res.stdout}\n{res.stderr}")
+
+
 def sources() -> list[Path]:
     return sorted(CSRC.glob("*.cu"))
 
@@ -71,7 +97,8 @@ def build(force: bool = False, verbose: bool = False, ptxas_v: bool = False) -> 
     if not srcs:
         raise RuntimeError(f"no CUDA sources under {CSRC}")
     logs = []
-    with cf.ThreadPoolExecutor(max_workers=min(len(srcs), os.cpu_count() or 4)) as ex:
+    with cf.ThreadPoolExecutor(max_workers=min(len(srcs) + 1, os.cpu_count() or 4)) as ex:
+        host = ex.submit(_build_host, force, verbose)
         futs = [ex.submit(_compile, s, force, verbose, ptxas_v) for s in srcs]
         objs = []
         for f in futs:
@@ -79,6 +106,7 @@ def build(force: bool = False, verbose: bool = False, ptxas_v: bool = False) -> 
             objs.append(o)
             if log:
                 logs.append(log)
+        host.result()
     if ptxas_v:
         print("\n".join(logs))
     need_link = force or not LIB.exists() or any(o.stat().st_mtime > LIB.stat().st_mtime for o in objs)

@@ -19,6 +19,10 @@ entry point here             reference entry it replaces
 
 Differences from the reference, all deliberate:
 
+* the entry points run on the native host path (``csrc/host/torch_host.cpp``: checks, allocation,
+  launch and the autograd node in C++); what it does not cover comes back as None and is handled
+  here, by the ``*_Func`` classes: arguments that are wrong (the exceptions are raised here), tensor
+  subclasses, channel strides other than 1, empty tensors, bias gradients, in-place rotation.
 * ``kernel_cache`` slots hold a validated launch key (shapes, strides, dtypes)
   instead of a compiled-kernel handle.  A call whose key differs re-validates
   and replaces the slot, so one module can be reused across shapes and dtypes
@@ -110,6 +114,20 @@ def _tracing() -> bool:
         from . import library  # noqa: F401  (registers torch.ops.rgd_b200.*)
         return True
     return False
+
+
+_HOST = None
+
+
+def _bind_host(t):
+    """The native host path, loaded on the first CUDA tensor.  None for anything else: the Python path
+    then raises (there is no CPU path)."""
+    global _HOST
+    if _HOST is None and isinstance(t, torch.Tensor) and t.is_cuda:
+        host = _lib.host()
+        host.set_single_pass(_ATTN_BWD_MODE == "single_pass")
+        _HOST = host
+    return _HOST
 
 
 def _needs_grad(*tensors) -> bool:
@@ -236,6 +254,11 @@ def triton_norm_func_fn(x, norm_eps=1e-6, use_ptx=False, kernel_cache=None):
     """L2-normalise the rows of x.  ``use_ptx`` is accepted and ignored."""
     if _tracing():
         return torch.ops.rgd_b200.l2norm([x], float(norm_eps))[0]
+    host = _HOST or _bind_host(x)
+    if host is not None:
+        out = host.rows(kernel_cache, norm_eps, False, x)
+        if out is not None:
+            return out
     if not _needs_grad(x):
         return _l2_forward([x], norm_eps, kernel_cache, "L2Normalize")[1][0]
     return Norm_Func.apply(x, norm_eps, use_ptx, kernel_cache)
@@ -263,6 +286,11 @@ def triton_fused_norm_func_fn(x1, x2, norm_eps=1e-6, kernel_cache=None):
     if _tracing():
         y1, y2 = torch.ops.rgd_b200.l2norm([x1, x2], float(norm_eps))
         return y1, y2
+    host = _HOST or _bind_host(x1)
+    if host is not None:
+        out = host.rows(kernel_cache, norm_eps, False, x1, x2)
+        if out is not None:
+            return out
     if not _needs_grad(x1, x2):
         ys = _l2_forward([x1, x2], norm_eps, kernel_cache, "FusedL2Normalize2")[1]
         return ys[0], ys[1]
@@ -384,6 +412,11 @@ class RMS_Func(torch.autograd.Function):
 def triton_rms_func_fn(x, w, norm_eps=1e-6, kernel_cache=None):
     if _tracing():
         return torch.ops.rgd_b200.rmsnorm([x], [w], float(norm_eps))[0]
+    host = _HOST or _bind_host(x)
+    if host is not None:
+        out = host.rows(kernel_cache, norm_eps, True, x, w)
+        if out is not None:
+            return out
     if not _needs_grad(x, w):
         return _rms_forward([x], [w], norm_eps, kernel_cache, "FusedRMSNorm")[2][0]
     return RMS_Func.apply(x, w, norm_eps, kernel_cache)
@@ -413,6 +446,11 @@ def triton_fused_rms_func_fn(x1, x2, w1, w2, norm_eps=1e-6, kernel_cache=None):
     if _tracing():
         y1, y2 = torch.ops.rgd_b200.rmsnorm([x1, x2], [w1, w2], float(norm_eps))
         return y1, y2
+    host = _HOST or _bind_host(x1)
+    if host is not None:
+        out = host.rows(kernel_cache, norm_eps, True, x1, x2, w1, w2)
+        if out is not None:
+            return out
     if not _needs_grad(x1, x2, w1, w2):
         ys = _rms_forward([x1, x2], [w1, w2], norm_eps, kernel_cache, "FusedRMSNorm2")[2]
         return ys[0], ys[1]
@@ -524,6 +562,11 @@ class Fused_LNQK_Func(torch.autograd.Function):
 def triton_fused_ln_func_fn(query, key, heads_second=True, norm_eps=1e-6, kernel_cache=None):
     if _tracing():
         return torch.ops.rgd_b200.headln(query, key, bool(heads_second), float(norm_eps))
+    host = _HOST or _bind_host(query)
+    if host is not None:
+        out = host.headln(kernel_cache, norm_eps, heads_second, query, key)
+        if out is not None:
+            return out
     if not _needs_grad(query, key):
         return _ln_forward(query, key, heads_second, norm_eps, kernel_cache)[2:]
     return Fused_LNQK_Func.apply(query, key, heads_second, norm_eps, kernel_cache)
@@ -605,6 +648,11 @@ def triton_rope_fn(query, key, pos_emb, seq_cutoff=None, heads_second=True, fuse
         nq, nk = (query.shape[2], key.shape[2]) if heads_second else (query.shape[1], key.shape[1])
         cq, ck = _cutoffs(seq_cutoff, nq, nk)
         return torch.ops.rgd_b200.rope(query, key, pos_emb, cq, ck, bool(heads_second), False)
+    host = _HOST or _bind_host(query)
+    if host is not None and not in_place:
+        out = host.rotary(kernel_cache, None, heads_second, query, key, pos_emb, seq_cutoff)
+        if out is not None:
+            return out
     if not _needs_grad(query, key, pos_emb):
         return _rope_forward(query, key, pos_emb, seq_cutoff, heads_second, in_place, kernel_cache)[4:]
     return CombinedRoPEFunc.apply(query, key, pos_emb, seq_cutoff, heads_second, in_place, kernel_cache)
@@ -673,6 +721,11 @@ def triton_fused_ln_rope_fn(query, key, pos_emb, seq_cutoff=None, heads_second=T
         nq, nk = (query.shape[2], key.shape[2]) if heads_second else (query.shape[1], key.shape[1])
         cq, ck = _cutoffs(seq_cutoff, nq, nk)
         return torch.ops.rgd_b200.lnrope(query, key, pos_emb, cq, ck, bool(heads_second), float(norm_eps))
+    host = _HOST or _bind_host(query)
+    if host is not None:
+        out = host.rotary(kernel_cache, norm_eps, heads_second, query, key, pos_emb, seq_cutoff)
+        if out is not None:
+            return out
     if not _needs_grad(query, key, pos_emb):
         return _lnrope_forward(query, key, pos_emb, seq_cutoff, heads_second, norm_eps, kernel_cache)[4:]
     return FusedRoPEFunc.apply(query, key, pos_emb, seq_cutoff, heads_second, norm_eps, kernel_cache)
@@ -776,6 +829,22 @@ def _bias_tiles(cache, bias, bias_t, bias_s, q, seqlen_q, seqlen_k, causal):
     return None
 
 
+def _native_tiles(cache, bias, q, k, causal):
+    """_bias_tiles for the native host path: the same policy, with the cheap refusals first so that an
+    ordinary call does not describe its bias twice."""
+    if (cache is None or causal or not _SKIP_MASKED_TILES or bias.ndim != 4 or q.ndim != 4 or k.ndim != 4
+            or bias.shape[2] == 1 or bias.dtype == torch.float32 or bias.requires_grad or bias.stride(-1) != 1
+            or not bias.is_cuda or tuple(bias.shape[2:]) != (q.shape[1], k.shape[1])
+            or ((q.shape[1] + 127) // 128) * ((k.shape[1] + 127) // 128) < _SKIP_MIN_TILES):
+        return None
+    ent = getattr(cache, "_tiles", None)
+    if ent is not None and ent[2] is not None and ent[0]() is bias and ent[1] == bias._version:
+        return ent[2] if torch.is_tensor(ent[2]) else None
+    _check_attn(q, k, k)
+    bias_t, bias_s = _prep_bias(bias, q, q.shape[1], k.shape[1])
+    return _bias_tiles(cache, bias, bias_t, bias_s, q, q.shape[1], k.shape[1], causal)
+
+
 def _attn_forward(q, k, v, bias, causal, softmax_scale, cache):
     q, k, v = _last_contig(q), _last_contig(k), _last_contig(v)
     plan = _plan(cache, "fwd", _key(q, k, v, bias, extra=("attn", bool(causal))), lambda: _check_attn(q, k, v))
@@ -839,6 +908,8 @@ def set_attention_backward(mode: str) -> str:
     global _ATTN_BWD_MODE
     _require(mode in ("single_pass", "two_kernel"), "mode must be 'single_pass' or 'two_kernel'")
     prev, _ATTN_BWD_MODE = _ATTN_BWD_MODE, mode
+    if _HOST is not None:
+        _HOST.set_single_pass(mode == "single_pass")
     return prev
 
 
@@ -930,6 +1001,12 @@ def flash_attn_func(q, k, v, bias=None, causal=False, softmax_scale=None, return
                               kernel_cache)
         o = res[0][..., :d].contiguous()
         return (o, res[1]) if return_lse else o
+    host = _HOST or _bind_host(q)
+    if host is not None:
+        tiles = _native_tiles(kernel_cache, bias, q, k, causal) if bias is not None else None
+        out = host.attn(kernel_cache, q, k, v, bias, tiles, causal, softmax_scale, return_lse)
+        if out is not None:
+            return out
     if not _needs_grad(q, k, v, bias):
         _, _, _, o, lse, _, _, _ = _attn_forward(q, k, v, bias, causal, softmax_scale, kernel_cache)
     else:

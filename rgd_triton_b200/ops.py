@@ -12,67 +12,62 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
+from . import _lib
 from . import functional as F_
 
 
 class _LaunchCache:
     """Named slots, one per kernel of an operator (``fwd``, ``bwd``, ...), plus
-    the native launch-plan cache of the C library.
+    the native launch state of the C library.
 
-    A slot holds the launch key (shapes, strides, dtypes, device) that was last
-    validated for that kernel; a call with the same key skips host-side
-    validation, a call with a different key re-validates and replaces it.
+    A slot is None until its kernel has run through this cache; then it holds what was
+    launched last: the native host path keeps shapes, strides and types in ``_state``, the
+    Python path the launch key it validated (a call with the same key skips validation, a call
+    with a different key re-validates and replaces it).
     ``native()`` is the ``rgd_cache`` handle (created on first use) in which the
     library keeps the encoded TMA descriptors of the calls this module made.
     """
 
+    _BACKWARD = ("bwd", "bwd_odot", "bwd_dw")
+
     def __init__(self, fields):
-        for name in fields:
-            setattr(self, name, None)
-        self._native = None
+        self._fields = tuple(fields)
+
+    def __getattr__(self, name):
+        # only reached for names that are not set on the object
+        if name == "_state":
+            state = _lib.host().LaunchState()
+            self.__dict__["_state"] = state
+            return state
+        if not name.startswith("_") and name in self.__dict__.get("_fields", ()):
+            state = self.__dict__.get("_state")
+            return None if state is None else state.seen(1 if name in self._BACKWARD else 0)
+        raise AttributeError(name)
 
     def native(self):
-        if self._native is None:
-            from . import _lib
-            self._native = _lib.load().rgd_cache_create()
-        return self._native
+        return self._state.native()
 
     def stats(self):
         """(hits, misses, entries) of the native descriptor cache."""
         import ctypes as C
-        from . import _lib
         h, m, e = C.c_int64(0), C.c_int64(0), C.c_int64(0)
-        if self._native is not None:
-            _lib.load().rgd_cache_stats(self._native, C.byref(h), C.byref(m), C.byref(e))
+        if "_state" in self.__dict__:
+            _lib.load().rgd_cache_stats(self.native(), C.byref(h), C.byref(m), C.byref(e))
         return h.value, m.value, e.value
 
-    def __del__(self):
-        native, self._native = getattr(self, "_native", None), None
-        if native is not None:
-            try:
-                from . import _lib
-                _lib.load().rgd_cache_destroy(native)
-            except Exception:       # interpreter shutdown
-                pass
-
-    # the native handle belongs to this process and this object only
+    # the native state belongs to this process and this object only
     # (the marshalled arguments kept under "_plan_*" hold raw pointers and "_tiles" the tile lists of
     # the last bias tensor: they stay behind too)
     def __getstate__(self):
-        state = {k: v for k, v in vars(self).items() if not k.startswith("_plan_") and k != "_tiles"}
-        state["_native"] = None
-        return state
+        return {k: v for k, v in vars(self).items() if not k.startswith("_plan_") and k not in ("_tiles", "_state")}
 
     def __deepcopy__(self, memo):
         new = _LaunchCache(())
-        for k, v in vars(self).items():
-            if not k.startswith("_plan_") and k != "_tiles":
-                setattr(new, k, None if k == "_native" else v)
+        new.__dict__.update(self.__getstate__())
         return new
 
     def __repr__(self):
-        slots = {k: v for k, v in vars(self).items() if not k.startswith("_")}
-        return "LaunchCache(" + ", ".join(f"{k}={'set' if v is not None else None}" for k, v in slots.items()) + ")"
+        return "LaunchCache(" + ", ".join(f"{k}={'set' if getattr(self, k) is not None else None}" for k in self._fields) + ")"
 
 
 class CachableModule(nn.Module):
