@@ -281,9 +281,9 @@ int64_t rgd_attn_bwd_workspace_bytes(int64_t B, int64_t H, int64_t Tq,
                                      int64_t Tk, int64_t d, int dtype);
 
 /* Scratch bytes that select the single-pass backward (0 where there is none:
- * it exists for head_dim 64 on the tensor-memory path, without tile lists and
+ * it exists for head_dim <= 64 on the tensor-memory path, without tile lists and
  * without a bias gradient): the bytes above, rounded up to 256, plus an fp32 dQ
- * accumulator of B * H * Tq (rounded up to 128) * d elements, which the entry
+ * accumulator of B * H * Tq (rounded up to 128) * 64 elements, which the entry
  * point zeroes itself.  Given at least this much 256-byte aligned workspace,
  * rgd_attn_bwd evaluates S, dP and the exponentials once per tile pair and adds
  * the dQ partial tiles into the accumulator with vector reductions, the scheme
@@ -333,8 +333,8 @@ int rgd_attn_bwd_dbias(const rgd_heads *q, const rgd_heads *k,
 
 /* Which attention implementation rgd_attn_fwd / rgd_attn_bwd take for these
  * views: 1 = tcgen05 / tensor-memory / TMA kernels, 0 = general mma.sync
- * kernels.  Evaluates exactly the test the entry points use (head_dim 64 or
- * 128, every view 16-byte addressable with positive strides on dimensions of
+ * kernels.  Evaluates exactly the test the entry points use (head_dim a
+ * multiple of 8, every view 16-byte addressable with positive strides on dimensions of
  * extent > 1, and for the forward softmax_scale > 0). */
 int rgd_attn_fwd_uses_tmem(const rgd_heads *q, const rgd_heads *k,
                            const rgd_heads *v, const rgd_heads *o, int64_t B,

@@ -1,5 +1,5 @@
 // extern "C" attention entry points: argument validation, path selection
-// (tensor-memory kernels for aligned head_dim 64 / 128, general mma.sync
+// (tensor-memory kernels for aligned head dims that are multiples of 8, general mma.sync
 // kernels otherwise) and workspace layout.
 #include "attn_mma.cuh"
 

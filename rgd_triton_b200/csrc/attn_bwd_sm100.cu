@@ -51,7 +51,9 @@ struct BwdTmaParams {
     CUtensorMap mbias64;                // the same tensor with box 64 keys x 64 queries (dK/dV sub-blocks)
     int bias_h0, bias_b0;               // bias broadcast over heads / batch: coordinate 0
     const float *lse2, *delta_s;        // [B, H, Tq128]: lse * log2(e) (+inf past Tq), delta * scale (0 past Tq)
+    TileOrder order;
     int H, Tq, Tk, Tq128, causal;
+    int d;                              // channels, a multiple of 8, at most D: the tiles are zero-filled up to D
     float scale, scale_log2;
     int *status;
     // bias gradient (null when not wanted): vector form fp32 [B, H, Tk], matrix form [B, H, Tq, Tk] in
@@ -120,7 +122,9 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_tmem(const __grid_con
     BwdTmaSmem<D, BSTAGES> &sm = *reinterpret_cast<BwdTmaSmem<D, BSTAGES> *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int blk = blockIdx.x, bh = blockIdx.y;
+    int blk, bh;
+    tile_of(p.order, blk, bh);
+    if (!DKDV && p.causal) blk = p.order.nblk - 1 - blk;   // heavy causal tiles first
     const int b = bh / p.H, h = bh - b * p.H;
     const int r0 = blk * BT;                               // first key (DKDV) or query (DQ) of this CTA
     // Range of looped blocks.
@@ -158,6 +162,10 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_tmem(const __grid_con
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tbase = sm.tmem_base;
+    if (DKDV) {
+        grid_wait();        // the row statistics are in place
+        grid_trigger();     // the dQ kernel needs nothing from this one: it may fill the SMs this grid leaves idle
+    }
 
     if (warp == 8) {
         // ------------------------------ TMA producer ------------------------------
@@ -517,6 +525,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_tmem(const __grid_con
                     if (row < limit) {
 #pragma unroll
                         for (int i = 0; i < 32; i += 8) {
+                            if (col + i >= p.d) break;
                             uint4 v;
                             v.x = pack16b<BF16>(__uint_as_float(r[i]), __uint_as_float(r[i + 1]));
                             v.y = pack16b<BF16>(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]));
@@ -533,6 +542,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_tmem(const __grid_con
     tc_fence_before_sync();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tbase, TMEM_COLS);
+    if (!DKDV && blockIdx.x == gridDim.x - 1) grid_wait();      // this grid ends after the dK/dV kernel, which it runs beside
 }
 
 // ---------------------------------------------------------------------------
@@ -587,7 +597,8 @@ __global__ void __launch_bounds__(DKDV_SUB_THREADS, 1) attn_bwd_dkdv_sub(const _
     Smem &sm = *reinterpret_cast<Smem *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int blk = blockIdx.x, bh = blockIdx.y;
+    int blk, bh;
+    tile_of(p.order, blk, bh);                             // the first key blocks are the heavy causal ones
     const int b = bh / p.H, h = bh - b * p.H;
     const int r0 = blk * BT;                               // first key of this CTA
     const int i_begin = p.causal ? r0 / BT : 0;
@@ -597,7 +608,7 @@ __global__ void __launch_bounds__(DKDV_SUB_THREADS, 1) attn_bwd_dkdv_sub(const _
     // in shared memory (sm.qblk) before the stage's barrier, where the compute threads pick it up.
     int tl_idx = -1;
     if constexpr (LISTS)
-        tl_idx = (int)(((p.bias_b0 ? 0 : b) * (p.bias_h0 ? 1 : p.H) + (p.bias_h0 ? 0 : h)) * (int)gridDim.x + blk);
+        tl_idx = (int)(((p.bias_b0 ? 0 : b) * (p.bias_h0 ? 1 : p.H) + (p.bias_h0 ? 0 : h)) * p.order.nblk + blk);
     const int nit = LISTS ? (int)p.tlk_cnt[LISTS ? tl_idx : 0] : max(i_end - i_begin, 0);
     const int nsub = 2 * nit;
     int *status = p.status;
@@ -627,6 +638,8 @@ __global__ void __launch_bounds__(DKDV_SUB_THREADS, 1) attn_bwd_dkdv_sub(const _
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tbase = sm.tmem_base;
+    grid_wait();            // the row statistics are in place
+    grid_trigger();         // the dQ kernel needs nothing from this one: it may fill the SMs this grid leaves idle
 
     if (warp == 8) {
         // ------------------------------ TMA producer ------------------------------
@@ -952,6 +965,7 @@ __global__ void __launch_bounds__(DKDV_SUB_THREADS, 1) attn_bwd_dkdv_sub(const _
                     if (row < p.Tk) {
 #pragma unroll
                         for (int i = 0; i < 32; i += 8) {
+                            if (cc + i >= p.d) break;
                             uint4 v;
                             v.x = pack16b<BF16>(__uint_as_float(r[i]), __uint_as_float(r[i + 1]));
                             v.y = pack16b<BF16>(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]));
@@ -1025,7 +1039,8 @@ __global__ void __launch_bounds__(SINGLE64_THREADS, 1) attn_bwd_single64(const _
     Smem &sm = *reinterpret_cast<Smem *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int blk = blockIdx.x, bh = blockIdx.y;
+    int blk, bh;
+    tile_of(p.order, blk, bh);                             // the first key blocks are the heavy causal ones
     const int b = bh / p.H, h = bh - b * p.H;
     const int r0 = blk * BT;                               // first key of this CTA
     const int i_begin = p.causal ? r0 / BT : 0;
@@ -1035,7 +1050,7 @@ __global__ void __launch_bounds__(SINGLE64_THREADS, 1) attn_bwd_single64(const _
     // in shared memory (sm.qblk) before the stage's barrier, where the compute threads pick it up.
     int tl_idx = -1;
     if constexpr (LISTS)
-        tl_idx = (int)(((p.bias_b0 ? 0 : b) * (p.bias_h0 ? 1 : p.H) + (p.bias_h0 ? 0 : h)) * (int)gridDim.x + blk);
+        tl_idx = (int)(((p.bias_b0 ? 0 : b) * (p.bias_h0 ? 1 : p.H) + (p.bias_h0 ? 0 : h)) * p.order.nblk + blk);
     const int nit = LISTS ? (int)p.tlk_cnt[LISTS ? tl_idx : 0] : max(i_end - i_begin, 0);
     const int nsub = 2 * nit;
     int *status = p.status;
@@ -1067,6 +1082,8 @@ __global__ void __launch_bounds__(SINGLE64_THREADS, 1) attn_bwd_single64(const _
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tbase = sm.tmem_base;
+    grid_wait();            // the row statistics and the zeroed accumulator are in place
+    grid_trigger();
 
     // Registers move from the helper and read-back warps to the compute warps (the launch gives every
     // thread 65536 / 512 = 128): each role's first instruction resizes its warpgroup.
@@ -1450,6 +1467,7 @@ __global__ void __launch_bounds__(SINGLE64_THREADS, 1) attn_bwd_single64(const _
                     if (row < p.Tk) {
 #pragma unroll
                         for (int i = 0; i < 32; i += 8) {
+                            if (cc + i >= p.d) break;
                             uint4 v;
                             v.x = pack16b<BF16>(__uint_as_float(r[i]), __uint_as_float(r[i + 1]));
                             v.y = pack16b<BF16>(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]));
@@ -1495,9 +1513,7 @@ struct alignas(1024) DqPipeSmem {
 };
 constexpr int DQ_PIPE_THREADS = 352;   // 8 compute warps, TMA producer, two MMA issuers
 
-// VEC: a vector bias (one value per key) is added to the scores; each compute thread fetches the
-// values of its 64 keys per block (the same for every query row, so they come from L1).
-template <int D, bool BF16, bool VEC>
+template <int D, bool BF16>
 __global__ void __launch_bounds__(DQ_PIPE_THREADS, 1) attn_bwd_dq_pipe(const __grid_constant__ BwdTmaParams p) {
     constexpr int HALVES = D / 64;
     constexpr uint32_t PANEL = 128 * 64 * 2;
@@ -1510,7 +1526,9 @@ __global__ void __launch_bounds__(DQ_PIPE_THREADS, 1) attn_bwd_dq_pipe(const __g
     DqPipeSmem<D> &sm = *reinterpret_cast<DqPipeSmem<D> *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int blk = blockIdx.x, bh = blockIdx.y;
+    int blk, bh;
+    tile_of(p.order, blk, bh);
+    if (p.causal) blk = p.order.nblk - 1 - blk;            // heavy causal tiles first
     const int b = bh / p.H, h = bh - b * p.H;
     const int r0 = blk * BT;                               // first query of this CTA
     const int i_end = ((p.causal ? min(p.Tk, r0 + BT) : p.Tk) + BT - 1) / BT;
@@ -1661,54 +1679,23 @@ __global__ void __launch_bounds__(DQ_PIPE_THREADS, 1) attn_bwd_dq_pipe(const __g
         const float lse_row = p.lse2[(int64_t)bh * p.Tq128 + row];
         const float dsc_row = p.delta_s[(int64_t)bh * p.Tq128 + row];
 
-        const char *bias_bh = nullptr;
-        if constexpr (VEC)
-            bias_bh = reinterpret_cast<const char *>(p.bias) +
-                      ((int64_t)b * p.b_sb + (int64_t)h * p.b_sh) * (p.bias_f32 ? 4 : 2);
-        // off[i] = bias * log2(e) - lse * log2(e) for the 32 keys starting at column c of this
-        // thread's 64 in block j (just -lse without a bias); keys past the end read as bias 0
-        auto offsets = [&](int j, int c, float *off) {
-            if constexpr (VEC) {
-                const int k0 = j * BT + half * 64 + c;
-                if (!p.bias_f32 && p.bias_vec && k0 + 32 <= p.Tk) {
-                    const T *src = reinterpret_cast<const T *>(bias_bh) + k0;
-#pragma unroll
-                    for (int q4 = 0; q4 < 4; ++q4) {
-                        const Vec<T, 8> v8 = load_vec<T, 8>(src + 8 * q4);
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) off[8 * q4 + e] = fmaf(to_f32<T>(v8.v[e]), LOG2E, -lse_row);
-                    }
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        float bvl = 0.f;
-                        if (k0 + i < p.Tk)
-                            bvl = p.bias_f32 ? reinterpret_cast<const float *>(bias_bh)[k0 + i]
-                                             : to_f32<T>(reinterpret_cast<const T *>(bias_bh)[k0 + i]);
-                        off[i] = fmaf(bvl, LOG2E, -lse_row);
-                    }
-                }
-            }
-        };
         // P of block j from its scores (32 columns starting at column c of this thread's 64)
         auto p_from_s = [&](const uint32_t (&r)[32], float *pv, int j, int c) {
             const int blk0 = j * BT;
-            float off[VEC ? 32 : 1];
-            offsets(j, c, off);
             // blocks that need per-element masking: the diagonal blocks under the causal mask
             // and the block touching the end of the keys
             const bool slow = (p.causal && blk0 + BT > r0) || blk0 + BT > p.Tk;
             if (!slow) {
 #pragma unroll
                 for (int i = 0; i < 32; ++i)
-                    pv[i] = ex2b(fmaf(__uint_as_float(r[i]), p.scale_log2, VEC ? off[VEC ? i : 0] : -lse_row));
+                    pv[i] = ex2b(fmaf(__uint_as_float(r[i]), p.scale_log2, -lse_row));
             } else {
                 const int c0 = blk0 + half * 64 + c;
 #pragma unroll
                 for (int i = 0; i < 32; ++i) {
                     const int kj = c0 + i;
                     const bool masked = kj >= p.Tk || row >= p.Tq || (p.causal && kj > row);
-                    pv[i] = masked ? 0.f : ex2b(fmaf(__uint_as_float(r[i]), p.scale_log2, VEC ? off[VEC ? i : 0] : -lse_row));
+                    pv[i] = masked ? 0.f : ex2b(fmaf(__uint_as_float(r[i]), p.scale_log2, -lse_row));
                 }
             }
         };
@@ -1756,18 +1743,14 @@ __global__ void __launch_bounds__(DQ_PIPE_THREADS, 1) attn_bwd_dq_pipe(const __g
                 }
                 uint32_t pk[16];
                 if (next && !slow_next) {
-                    float off[VEC ? 32 : 1];
-                    offsets(it + 1, 32 * c, off);
                     // element by element, so that the exponentials of the next block (MUFU) and
                     // the dS arithmetic of this one (FMA pipe) issue side by side
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
                         const float a0 = pv[32 * c + 2 * i] * fmaf(__uint_as_float(ga[2 * i]), p.scale, -dsc_row);
                         const float a1 = pv[32 * c + 2 * i + 1] * fmaf(__uint_as_float(ga[2 * i + 1]), p.scale, -dsc_row);
-                        pv[32 * c + 2 * i] = ex2b(fmaf(__uint_as_float(ra[2 * i]), p.scale_log2,
-                                                       VEC ? off[VEC ? 2 * i : 0] : -lse_row));
-                        pv[32 * c + 2 * i + 1] = ex2b(fmaf(__uint_as_float(ra[2 * i + 1]), p.scale_log2,
-                                                           VEC ? off[VEC ? 2 * i + 1 : 0] : -lse_row));
+                        pv[32 * c + 2 * i] = ex2b(fmaf(__uint_as_float(ra[2 * i]), p.scale_log2, -lse_row));
+                        pv[32 * c + 2 * i + 1] = ex2b(fmaf(__uint_as_float(ra[2 * i + 1]), p.scale_log2, -lse_row));
                         pk[i] = pack16b<BF16>(a0, a1);
                     }
                     // packed dS of chunk c goes to columns [c*16, c*16+16) of this thread's 64, all read already
@@ -1807,6 +1790,7 @@ __global__ void __launch_bounds__(DQ_PIPE_THREADS, 1) attn_bwd_dq_pipe(const __g
                 if (row < p.Tq) {
 #pragma unroll
                     for (int i = 0; i < 32; i += 8) {
+                        if (col + i >= p.d) break;
                         uint4 v;
                         v.x = pack16b<BF16>(__uint_as_float(r[i]), __uint_as_float(r[i + 1]));
                         v.y = pack16b<BF16>(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]));
@@ -1822,6 +1806,7 @@ __global__ void __launch_bounds__(DQ_PIPE_THREADS, 1) attn_bwd_dq_pipe(const __g
     tc_fence_before_sync();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tbase, TMEM_COLS);
+    if (blockIdx.x == gridDim.x - 1) grid_wait();      // this grid ends after the dK/dV kernel, which it runs beside
 }
 
 // ---------------------------------------------------------------------------
@@ -1853,10 +1838,14 @@ struct alignas(1024) DqBiasSmem {
     uint32_t tmem_base;
 };
 
-// VEC: the bias is a vector (one value per key, 16-bit, 16-byte addressable, key count a multiple of 8):
-// the producer stages the block's 128 values (256 bytes) with one bulk copy instead of a 32 KB tile, and
-// every compute thread reads its 64 from shared memory (the same addresses in all threads: broadcasts).
-template <int D, bool BF16, bool DBIAS, bool LISTS, bool VEC>
+// VEC: the bias is a vector (one value per key), staged per key block in shared memory, where every
+// thread reads its 64 values at the same addresses as all others (broadcasts):
+//   1  16-bit, 16-byte addressable, key count a multiple of 8: one 256-byte bulk copy by the producer
+//   2  any other: the compute threads (thread = key) load the next block's values while they form dS of
+//      this one and leave them as fp32.  6 % slower than 1 at [2, 4608, 24, 128] (1.81 against 1.71 ms of
+//      backward), but fetching unaligned values per thread from global memory, as the unfused loop did,
+//      took twice the time (224 -> 124 us at [2, 1100, 12, 128]).
+template <int D, bool BF16, bool DBIAS, bool LISTS, int VEC>
 __global__ void __launch_bounds__(DQ_PIPE_THREADS, 1) attn_bwd_dq_bias(const __grid_constant__ BwdTmaParams p,
                                                                        const void *q_base, const void *do_base,
                                                                        int64_t q_sb, int64_t q_sh, int64_t q_sn,
@@ -1874,7 +1863,9 @@ __global__ void __launch_bounds__(DQ_PIPE_THREADS, 1) attn_bwd_dq_bias(const __g
     DqBiasSmem<D> &sm = *reinterpret_cast<DqBiasSmem<D> *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int blk = blockIdx.x, bh = blockIdx.y;
+    int blk, bh;
+    tile_of(p.order, blk, bh);
+    if (p.causal) blk = p.order.nblk - 1 - blk;            // heavy causal tiles first
     const int b = bh / p.H, h = bh - b * p.H;
     const int r0 = blk * BT;                               // first query of this CTA
     const int i_end = ((p.causal ? min(p.Tk, r0 + BT) : p.Tk) + BT - 1) / BT;
@@ -1884,7 +1875,7 @@ __global__ void __launch_bounds__(DQ_PIPE_THREADS, 1) attn_bwd_dq_bias(const __g
     const uint16_t *tl = nullptr;
     if constexpr (LISTS) {
         const int64_t slice = (int64_t)(p.bias_b0 ? 0 : b) * (p.bias_h0 ? 1 : p.H) + (p.bias_h0 ? 0 : h);
-        const int64_t idx = slice * gridDim.x + blk;
+        const int64_t idx = slice * p.order.nblk + blk;
         tl = p.tlq_list + idx * p.tl_nkb;
         nit = p.tlq_cnt[idx];
     }
@@ -1905,7 +1896,7 @@ __global__ void __launch_bounds__(DQ_PIPE_THREADS, 1) attn_bwd_dq_bias(const __g
         for (int s = 0; s < 2; ++s) {
             mbar_init(&sm.v_full[s], 1);
             mbar_init(&sm.v_empty[s], 1);
-            mbar_init(&sm.bb_full[s], 1);
+            mbar_init(&sm.bb_full[s], VEC == 2 ? 128 : 1);
             mbar_init(&sm.bb_empty[s], 256);
         }
         fence_mbar_init();
@@ -1924,7 +1915,7 @@ __global__ void __launch_bounds__(DQ_PIPE_THREADS, 1) attn_bwd_dq_bias(const __g
         if (lane == 0 && nit > 0) {
             tma_prefetch_desc(&p.mk);
             tma_prefetch_desc(&p.mv);
-            if constexpr (!VEC) tma_prefetch_desc(&p.mbias);
+            if constexpr (VEC == 0) tma_prefetch_desc(&p.mbias);
             bool ok = true;
             int ks = 0;
             uint32_t kph = 0;                              // phase of the K ring slot's previous use
@@ -1937,15 +1928,17 @@ __global__ void __launch_bounds__(DQ_PIPE_THREADS, 1) attn_bwd_dq_bias(const __g
                     tma_load_4d(sm.k[ks] + hh * PANEL, &p.mk, &sm.k_full[ks], hh * 64, row, h, b);
                 if (++ks == 3) { ks = 0; kph ^= 1u; }
                 const int vs = it & 1;
-                // bias tile of block it: rows = this CTA's queries, columns = the block's keys
-                ok = mbar_wait(&sm.bb_empty[vs], ((uint32_t)(it >> 1) & 1u) ^ 1u, status, 43);
-                if (!ok) break;
-                if constexpr (VEC) {
+                if constexpr (VEC == 1) {
+                    ok = mbar_wait(&sm.bb_empty[vs], ((uint32_t)(it >> 1) & 1u) ^ 1u, status, 43);
+                    if (!ok) break;
                     const uint32_t nbytes = (uint32_t)min(BT, p.Tk - row) * 2u;       // a multiple of 16
                     mbar_expect_tx(&sm.bb_full[vs], nbytes);
                     bulk_load_1d(sm.bias[vs], reinterpret_cast<const char *>(p.bias) +
                                                   ((int64_t)b * p.b_sb + (int64_t)h * p.b_sh + row) * 2, nbytes, &sm.bb_full[vs]);
-                } else {
+                } else if constexpr (VEC == 0) {
+                    // bias tile of block it: rows = this CTA's queries, columns = the block's keys
+                    ok = mbar_wait(&sm.bb_empty[vs], ((uint32_t)(it >> 1) & 1u) ^ 1u, status, 43);
+                    if (!ok) break;
                     mbar_expect_tx(&sm.bb_full[vs], BIAS_BYTES);
                     for (int pn = 0; pn < 2; ++pn)
                         tma_load_4d(sm.bias[vs] + pn * (BT * 128), &p.mbias, &sm.bb_full[vs], row + pn * 64, r0,
@@ -2051,7 +2044,7 @@ __global__ void __launch_bounds__(DQ_PIPE_THREADS, 1) attn_bwd_dq_bias(const __g
 #pragma unroll
                 for (int i = 0; i < ACOLS; i += 4) {
                     uint4 v = make_uint4(0u, 0u, 0u, 0u);
-                    if (row < p.Tq) v = __ldg(reinterpret_cast<const uint4 *>(src) + (i >> 2));
+                    if (row < p.Tq && half * (D / 2) + 2 * i < p.d) v = __ldg(reinterpret_cast<const uint4 *>(src) + (i >> 2));
                     a[i] = v.x; a[i + 1] = v.y; a[i + 2] = v.z; a[i + 3] = v.w;
                 }
                 const uint32_t dst = lane_base + (op == 0 ? QA_COL : DOA_COL) + half * ACOLS;
@@ -2070,19 +2063,44 @@ __global__ void __launch_bounds__(DQ_PIPE_THREADS, 1) attn_bwd_dq_bias(const __g
         // P of block j from this thread's 64 scores and its row of the block's bias tile; the
         // score columns are released as soon as they are in registers
         float pv[64];
+        // vector bias: the value of key row_l of block j (0 past the end of the keys, which is masked below)
+        const char *bias_bh = reinterpret_cast<const char *>(p.bias) + ((int64_t)b * p.b_sb + (int64_t)h * p.b_sh) * (p.bias_f32 ? 4 : 2);
+        auto vec_value = [&](int j) -> float {
+            const int kj = j * BT + row_l;
+            if (half != 0 || kj >= p.Tk) return 0.f;
+            return p.bias_f32 ? reinterpret_cast<const float *>(bias_bh)[kj] : to_f32<T>(reinterpret_cast<const T *>(bias_bh)[kj]);
+        };
+        auto vec_stage = [&](int j, float v) -> bool {
+            if (half != 0) return true;
+            if (!mbar_wait(&sm.bb_empty[j & 1], ((uint32_t)(j >> 1) & 1u) ^ 1u, status, 66)) return false;
+            reinterpret_cast<float *>(sm.bias[j & 1])[row_l] = v;
+            mbar_arrive(&sm.bb_full[j & 1]);
+            return true;
+        };
         auto load_p = [&](int j) -> bool {
             if (!mbar_wait(&sm.bb_full[j & 1], (uint32_t)(j >> 1) & 1u, status, 65)) return false;
             // 64 key columns = the whole 128-byte row of panel `half`; pv first holds
             // bias * log2(e) - lse * log2(e)
-            // (vector bias: the 64 values of this half of the block, the same for every row; values past
-            // the end of the keys were not loaded and are masked below)
-            const unsigned char *rowp = VEC ? sm.bias[j & 1] + half * 128 : sm.bias[j & 1] + half * (BT * 128) + row_l * 128;
+            if constexpr (VEC == 2) {
+                const float4 *src = reinterpret_cast<const float4 *>(sm.bias[j & 1]) + half * 16;
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                union { uint4 u; T v[8]; } cv;
-                cv.u = *reinterpret_cast<const uint4 *>(rowp + (VEC ? (c << 4) : ((c ^ (row_l & 7)) << 4)));
+                for (int c = 0; c < 16; ++c) {
+                    const float4 v = src[c];
+                    pv[4 * c] = fmaf(v.x, LOG2E, -lse_row);
+                    pv[4 * c + 1] = fmaf(v.y, LOG2E, -lse_row);
+                    pv[4 * c + 2] = fmaf(v.z, LOG2E, -lse_row);
+                    pv[4 * c + 3] = fmaf(v.w, LOG2E, -lse_row);
+                }
+            } else {
+                // (VEC == 1: values past the end of the keys were not loaded and are masked below)
+                const unsigned char *rowp = VEC ? sm.bias[j & 1] + half * 128 : sm.bias[j & 1] + half * (BT * 128) + row_l * 128;
 #pragma unroll
-                for (int e = 0; e < 8; ++e) pv[8 * c + e] = fmaf(to_f32<T>(cv.v[e]), LOG2E, -lse_row);
+                for (int c = 0; c < 8; ++c) {
+                    union { uint4 u; T v[8]; } cv;
+                    cv.u = *reinterpret_cast<const uint4 *>(rowp + (VEC ? (c << 4) : ((c ^ (row_l & 7)) << 4)));
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) pv[8 * c + e] = fmaf(to_f32<T>(cv.v[e]), LOG2E, -lse_row);
+                }
             }
             if (!mbar_wait(&sm.g1_full, (uint32_t)j & 1u, status, 60)) return false;
             tc_fence_after_sync();
@@ -2115,8 +2133,12 @@ __global__ void __launch_bounds__(DQ_PIPE_THREADS, 1) attn_bwd_dq_bias(const __g
             return true;
         };
 
-        bool ok = nit > 0 ? load_p(0) : true;
+        bool ok = true;
+        if (VEC == 2 && nit > 0) ok = vec_stage(0, vec_value(0));
+        if (ok && nit > 0) ok = load_p(0);
         for (int it = 0; it < nit && ok; ++it) {
+            float next_value = 0.f;
+            if (VEC == 2 && it + 1 < nit) next_value = vec_value(it + 1);
             // dS of block it
             ok = mbar_wait(&sm.g2_full, (uint32_t)it & 1u, status, 62);
             if (!ok) break;
@@ -2170,7 +2192,8 @@ __global__ void __launch_bounds__(DQ_PIPE_THREADS, 1) attn_bwd_dq_bias(const __g
             mbar_arrive(&sm.ds_ready);
             mbar_arrive(&sm.bb_empty[it & 1]);      // dS depends on every value read from the bias tile of block it
             // P of block it + 1, while the tensor pipe runs dQ(it) and dP(it + 1)
-            if (it + 1 < nit) ok = load_p(it + 1);
+            if (VEC == 2 && it + 1 < nit) ok = vec_stage(it + 1, next_value);
+            if (ok && it + 1 < nit) ok = load_p(it + 1);
         }
 
         // epilogue: dQ -> global
@@ -2192,6 +2215,7 @@ __global__ void __launch_bounds__(DQ_PIPE_THREADS, 1) attn_bwd_dq_bias(const __g
                 if (row < p.Tq) {
 #pragma unroll
                     for (int i = 0; i < 32; i += 8) {
+                        if (col + i >= p.d) break;
                         uint4 v;
                         v.x = pack16b<BF16>(__uint_as_float(r[i]), __uint_as_float(r[i + 1]));
                         v.y = pack16b<BF16>(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]));
@@ -2207,6 +2231,7 @@ __global__ void __launch_bounds__(DQ_PIPE_THREADS, 1) attn_bwd_dq_bias(const __g
     tc_fence_before_sync();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tbase, TMEM_COLS);
+    if (blockIdx.x == gridDim.x - 1) grid_wait();      // this grid ends after the dK/dV kernel, which it runs beside
 }
 
 // ---------------------------------------------------------------------------
@@ -2219,8 +2244,9 @@ __global__ void __launch_bounds__(DQ_PIPE_THREADS, 1) attn_bwd_dq_bias(const __g
 // dQ.  One CTA per 64 queries of one (batch, head): thread = (query, 16 channels).
 template <bool BF16>
 __global__ void __launch_bounds__(256) attn_bwd_dq_round64_kernel(const float *__restrict__ acc, void *dq, int64_t sb, int64_t sh,
-                                                                  int64_t sn, int H, int Tq, int Tq128) {
+                                                                  int64_t sn, int H, int Tq, int Tq128, int d) {
     using T = typename std::conditional<BF16, __nv_bfloat16, __half>::type;
+    grid_wait();
     const int bh = blockIdx.y, b = bh / H, h = bh - b * H;
     const int q = blockIdx.x * 64 + ((int)threadIdx.x & 63), part = (int)threadIdx.x >> 6;   // channels 16 part .. + 15
     if (q >= Tq) return;
@@ -2233,28 +2259,38 @@ __global__ void __launch_bounds__(256) attn_bwd_dq_round64_kernel(const float *_
         w[2 * g + 1] = pack16b<BF16>(v.z, v.w);
     }
     T *orow = reinterpret_cast<T *>(dq) + (int64_t)b * sb + (int64_t)h * sh + (int64_t)q * sn + part * 16;
-    *reinterpret_cast<uint4 *>(orow) = make_uint4(w[0], w[1], w[2], w[3]);
-    *reinterpret_cast<uint4 *>(orow + 8) = make_uint4(w[4], w[5], w[6], w[7]);
+    if (part * 16 < d) *reinterpret_cast<uint4 *>(orow) = make_uint4(w[0], w[1], w[2], w[3]);
+    if (part * 16 + 8 < d) *reinterpret_cast<uint4 *>(orow + 8) = make_uint4(w[4], w[5], w[6], w[7]);
 }
 
 template <typename T>
 __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __grid_constant__ AttnParams p, float *lse2, float *delta_s,
-                                                            int Tq128) {
-    // d / 8 lanes per row (d is 64 or 128, rows 16-byte aligned): 2 or 4 rows per warp
-    const int lpr = p.d >> 3;
+                                                            float *dq_acc, int Tq128) {
+    grid_trigger();          // the main kernel may set itself up meanwhile; it waits for this grid before it reads
+    // 8 or 16 lanes per row, 8 channels each (rows 16-byte aligned): 4 or 2 rows per warp
+    const int lpr = p.d > 64 ? 16 : 8;
     const int rows_per_cta = 256 / lpr;
     const int i = blockIdx.x * rows_per_cta + (int)threadIdx.x / lpr;
     const int l = (int)threadIdx.x % lpr;
     const int bh = blockIdx.y;
     const int b = bh / p.H, h = bh - b * p.H;
     float a = 0.f;
-    if (i < p.Tq) {
+    if (i < p.Tq && l * 8 < p.d) {
         const T *o = reinterpret_cast<const T *>(p.o) + (int64_t)b * p.o_sb + (int64_t)h * p.o_sh + (int64_t)i * p.o_sn;
         const T *g = reinterpret_cast<const T *>(p.d_o) + (int64_t)b * p.do_sb + (int64_t)h * p.do_sh +
                      (int64_t)i * p.do_sn;
         const Vec<T, 8> ov = load_vec_stream<T, 8>(o + l * 8), gv = load_vec<T, 8>(g + l * 8);
 #pragma unroll
         for (int e = 0; e < 8; ++e) a += to_f32<T>(ov.v[e]) * to_f32<T>(gv.v[e]);
+    }
+    // single-pass form (d <= 64, 32 rows per CTA, Tq128 a multiple of that): zero these rows of the dQ accumulator
+    if (dq_acc != nullptr) {
+        float4 *acc = reinterpret_cast<float4 *>(dq_acc) + (int64_t)bh * 16 * Tq128 + blockIdx.x * 32;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int t = (int)threadIdx.x + j * 256;
+            acc[(int64_t)(t >> 5) * Tq128 + (t & 31)] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
     }
     a = warp_group_sum(a, lpr);
     if (l == 0 && i < Tq128) {
@@ -2278,13 +2314,13 @@ int64_t single_pass_acc_offset(int64_t B, int64_t H, int64_t Tq) {
     return (tmem_bwd_workspace_bytes(B, H, Tq) + 255) / 256 * 256;
 }
 int64_t single_pass_acc_bytes(int64_t B, int64_t H, int64_t Tq, int64_t d) {
-    if (d != 64) return 0;
+    if (d < 8 || d > 64 || d % 8 != 0) return 0;
     const int64_t Tq128 = (Tq + 127) / 128 * 128;
-    return B * H * Tq128 * d * (int64_t)sizeof(float);
+    return B * H * Tq128 * 64 * (int64_t)sizeof(float);
 }
 
 bool tmem_bwd_eligible(const AttnParams &p) {
-    return (p.d == 64 || p.d == 128) && p.Tq >= 1 && p.Tk >= 1 && p.vec_q && p.vec_k && p.vec_v && p.vec_o && p.vec_do &&
+    return p.d >= 8 && p.d <= 128 && p.d % 8 == 0 && p.Tq >= 1 && p.Tk >= 1 && p.vec_q && p.vec_k && p.vec_v && p.vec_o && p.vec_do &&
            p.vec_dq && p.vec_dk && p.vec_dv && heads_map_encodable(p.q, p.B, p.H, p.Tq, p.q_sb, p.q_sh, p.q_sn) &&
            heads_map_encodable(p.k, p.B, p.H, p.Tk, p.k_sb, p.k_sh, p.k_sn) &&
            heads_map_encodable(p.v, p.B, p.H, p.Tk, p.v_sb, p.v_sh, p.v_sn) &&
@@ -2292,130 +2328,88 @@ bool tmem_bwd_eligible(const AttnParams &p) {
 }
 
 template <int D, bool BF16, bool DKDV, int BIAS>
-static int launch_bwd_one(const BwdTmaParams &bp, int nblocks, int BH, cudaStream_t st) {
+static int launch_bwd_one(const BwdTmaParams &bp, cudaStream_t st) {
     constexpr int BSTAGES = BIAS == 2 ? (D == 64 ? 2 : 1) : 0;
     const size_t smem = sizeof(BwdTmaSmem<D, BSTAGES>) + 1024;
     if (int e = ensure_dyn_smem(reinterpret_cast<const void *>(attn_bwd_tmem<D, BF16, DKDV, BIAS>), smem)) return e;
-    dim3 grid(nblocks, BH);
-    attn_bwd_tmem<D, BF16, DKDV, BIAS><<<grid, BWD_THREADS, smem, st>>>(bp);
-    count_launch();
-    return check_launch();
+    return launch_pdl(attn_bwd_tmem<D, BF16, DKDV, BIAS>, bp.order.nblk * bp.order.BH, BWD_THREADS, smem, st, bp);
 }
 
 template <int D, bool BF16, bool DKDV>
-static int launch_bwd_tmem(const BwdTmaParams &bp, int nblocks, int BH, cudaStream_t st) {
-    if (bp.bias_kind != RGD_BIAS_NONE && bp.bias_vec == 2) return launch_bwd_one<D, BF16, DKDV, 2>(bp, nblocks, BH, st);
-    if (bp.bias_kind != RGD_BIAS_NONE) return launch_bwd_one<D, BF16, DKDV, 1>(bp, nblocks, BH, st);
-    return launch_bwd_one<D, BF16, DKDV, 0>(bp, nblocks, BH, st);
+static int launch_bwd_tmem(const BwdTmaParams &bp, cudaStream_t st) {
+    if (bp.bias_kind != RGD_BIAS_NONE && bp.bias_vec == 2) return launch_bwd_one<D, BF16, DKDV, 2>(bp, st);
+    if (bp.bias_kind != RGD_BIAS_NONE) return launch_bwd_one<D, BF16, DKDV, 1>(bp, st);
+    return launch_bwd_one<D, BF16, DKDV, 0>(bp, st);
 }
 
 template <int D, bool BF16, int BIASM>
-static int launch_dkdv_sub(const BwdTmaParams &bp, int nblocks, int BH, cudaStream_t st) {
+static int launch_dkdv_sub(const BwdTmaParams &bp, cudaStream_t st) {
     const size_t smem = sizeof(DkdvSubSmem<D, BIASM == 1 || BIASM == 3>) + 1024;
     if (int e = ensure_dyn_smem(reinterpret_cast<const void *>(attn_bwd_dkdv_sub<D, BF16, BIASM>), smem)) return e;
-    dim3 grid(nblocks, BH);
-    attn_bwd_dkdv_sub<D, BF16, BIASM><<<grid, DKDV_SUB_THREADS, smem, st>>>(bp);
-    count_launch();
-    return check_launch();
+    return launch_pdl(attn_bwd_dkdv_sub<D, BF16, BIASM>, bp.order.nblk * bp.order.BH, DKDV_SUB_THREADS, smem, st, bp);
 }
 
 // Single-pass form (head_dim 64): zero the accumulator, one kernel for dK, dV and the dQ partial sums,
 // round dQ.  bias_mode: 0 none, 1 matrix bias staged by TMA, 2 vector bias.
 template <bool BF16>
-static int bwd_single64(BwdTmaParams &bp, const AttnParams &p, int bias_mode, cudaStream_t st) {
-    const int BH = p.B * p.H;
-    if (cudaMemsetAsync(bp.dq_acc, 0, (size_t)BH * bp.Tq128 * 64 * sizeof(float), st) != cudaSuccess) return RGD_E_DEVICE;
+static int bwd_single64(const BwdTmaParams &bp, const AttnParams &p, int bias_mode, cudaStream_t st) {
     const size_t smem = (bias_mode == 1 ? sizeof(Single64Smem<true>) : sizeof(Single64Smem<false>)) + 1024;
-    const void *kernel = bias_mode == 1   ? reinterpret_cast<const void *>(attn_bwd_single64<BF16, 1>)
-                         : bias_mode == 2 ? reinterpret_cast<const void *>(attn_bwd_single64<BF16, 2>)
-                                          : reinterpret_cast<const void *>(attn_bwd_single64<BF16, 0>);
-    if (int e = ensure_dyn_smem(kernel, smem)) return e;
-    dim3 grid((p.Tk + BT - 1) / BT, BH);
-    if (bias_mode == 1) attn_bwd_single64<BF16, 1><<<grid, SINGLE64_THREADS, smem, st>>>(bp);
-    else if (bias_mode == 2) attn_bwd_single64<BF16, 2><<<grid, SINGLE64_THREADS, smem, st>>>(bp);
-    else attn_bwd_single64<BF16, 0><<<grid, SINGLE64_THREADS, smem, st>>>(bp);
-    count_launch();
-    if (int e = check_launch()) return e;
-    dim3 rgrid((p.Tq + 63) / 64, BH);
-    attn_bwd_dq_round64_kernel<BF16><<<rgrid, 256, 0, st>>>(bp.dq_acc, p.dq, p.dq_sb, p.dq_sh, p.dq_sn, p.H, p.Tq, bp.Tq128);
-    count_launch();
-    return check_launch();
+    auto kernel = bias_mode == 1 ? attn_bwd_single64<BF16, 1> : bias_mode == 2 ? attn_bwd_single64<BF16, 2> : attn_bwd_single64<BF16, 0>;
+    if (int e = ensure_dyn_smem(reinterpret_cast<const void *>(kernel), smem)) return e;
+    if (int e = launch_pdl(kernel, bp.order.nblk * bp.order.BH, SINGLE64_THREADS, smem, st, bp)) return e;
+    return launch_pdl(attn_bwd_dq_round64_kernel<BF16>, dim3((p.Tq + 63) / 64, p.B * p.H), 256, 0, st, bp.dq_acc, p.dq, p.dq_sb,
+                      p.dq_sh, p.dq_sn, p.H, p.Tq, bp.Tq128, p.d);
 }
 
 template <int D, bool BF16>
 static int bwd_both(BwdTmaParams &bp, const AttnParams &p, cudaStream_t st) {
     const int BH = p.B * p.H;
+    // dK/dV kernel: the key blocks of a head share its Q and dO; dQ kernel: the query blocks its K and V
+    bp.order = make_tile_order((p.Tk + BT - 1) / BT, BH, p.causal, (int64_t)p.Tq * p.d * 4);
     bp.out1 = p.dv; bp.o1_sb = p.dv_sb; bp.o1_sh = p.dv_sh; bp.o1_sn = p.dv_sn;
     bp.out2 = p.dk; bp.o2_sb = p.dk_sb; bp.o2_sh = p.dk_sh; bp.o2_sn = p.dk_sn;
     if constexpr (D == 64) {
-        // the caller gave room for the fp32 dQ accumulator: single-pass form (not with tile lists or
-        // a bias gradient, which the two-kernel form serves)
-        if (bp.dq_acc != nullptr && bp.dbias == nullptr && bp.tlk_cnt == nullptr && p.Tk > 0) {
+        if (bp.dq_acc != nullptr) {
             if (bp.bias_kind == RGD_BIAS_NONE) return bwd_single64<BF16>(bp, p, 0, st);
-            if (bp.bias_vec == 2) return bwd_single64<BF16>(bp, p, 1, st);
-            if (bp.bias_kind == RGD_BIAS_VECTOR) return bwd_single64<BF16>(bp, p, 2, st);
+            return bwd_single64<BF16>(bp, p, bp.bias_vec == 2 ? 1 : 2, st);
         }
     }
     if (bp.bias_kind == RGD_BIAS_NONE) {
-        if (int e = launch_dkdv_sub<D, BF16, 0>(bp, (p.Tk + BT - 1) / BT, BH, st)) return e;
+        if (int e = launch_dkdv_sub<D, BF16, 0>(bp, st)) return e;
     } else if (bp.bias_vec == 2) {       // matrix bias staged by TMA, with or without tile lists
         if (bp.tlk_cnt != nullptr) {
-            if (int e = launch_dkdv_sub<D, BF16, 3>(bp, (p.Tk + BT - 1) / BT, BH, st)) return e;
-        } else if (int e = launch_dkdv_sub<D, BF16, 1>(bp, (p.Tk + BT - 1) / BT, BH, st)) {
+            if (int e = launch_dkdv_sub<D, BF16, 3>(bp, st)) return e;
+        } else if (int e = launch_dkdv_sub<D, BF16, 1>(bp, st)) {
             return e;
         }
     } else if (bp.bias_kind == RGD_BIAS_VECTOR) {
-        if (int e = launch_dkdv_sub<D, BF16, 2>(bp, (p.Tk + BT - 1) / BT, BH, st)) return e;
-    } else if (int e = launch_bwd_tmem<D, BF16, true>(bp, (p.Tk + BT - 1) / BT, BH, st)) {
+        if (int e = launch_dkdv_sub<D, BF16, 2>(bp, st)) return e;
+    } else if (int e = launch_bwd_tmem<D, BF16, true>(bp, st)) {
         return e;
     }
+    bp.order = make_tile_order((p.Tq + BT - 1) / BT, BH, p.causal, (int64_t)p.Tk * p.d * 4);
     bp.out1 = p.dq; bp.o1_sb = p.dq_sb; bp.o1_sh = p.dq_sh; bp.o1_sn = p.dq_sn;
     bp.out2 = nullptr;
-    if (bp.bias_kind == RGD_BIAS_VECTOR && bp.bias_vec == 1 && !bp.bias_f32 && p.Tk % 8 == 0) {
-        // 16-bit vector bias, 16-byte addressable: staged per key block by one bulk copy
-        const size_t smem = sizeof(DqBiasSmem<D>) + 1024;
-        const void *kernel = reinterpret_cast<const void *>(attn_bwd_dq_bias<D, BF16, false, false, true>);
-        if (int e = ensure_dyn_smem(kernel, smem)) return e;
-        dim3 grid((p.Tq + BT - 1) / BT, BH);
-        attn_bwd_dq_bias<D, BF16, false, false, true><<<grid, DQ_PIPE_THREADS, smem, st>>>(bp, p.q, p.d_o, p.q_sb, p.q_sh, p.q_sn,
-                                                                                             p.do_sb, p.do_sh, p.do_sn);
-        count_launch();
-        return check_launch();
-    }
-    if (bp.bias_kind == RGD_BIAS_NONE || (bp.bias_kind == RGD_BIAS_VECTOR && bp.bias_vec != 2)) {
-        const bool vec = bp.bias_kind == RGD_BIAS_VECTOR;
+    if (bp.bias_kind == RGD_BIAS_NONE) {
         const size_t smem = sizeof(DqPipeSmem<D>) + 1024;
-        const void *kernel = vec ? reinterpret_cast<const void *>(attn_bwd_dq_pipe<D, BF16, true>)
-                                 : reinterpret_cast<const void *>(attn_bwd_dq_pipe<D, BF16, false>);
-        if (int e = ensure_dyn_smem(kernel, smem)) return e;
-        dim3 grid((p.Tq + BT - 1) / BT, BH);
-        if (vec) attn_bwd_dq_pipe<D, BF16, true><<<grid, DQ_PIPE_THREADS, smem, st>>>(bp);
-        else attn_bwd_dq_pipe<D, BF16, false><<<grid, DQ_PIPE_THREADS, smem, st>>>(bp);
-        count_launch();
-        return check_launch();
+        auto kernel = attn_bwd_dq_pipe<D, BF16>;
+        if (int e = ensure_dyn_smem(reinterpret_cast<const void *>(kernel), smem)) return e;
+        return launch_pdl(kernel, bp.order.nblk * BH, DQ_PIPE_THREADS, smem, st, bp);
     }
-    if (bp.bias_vec == 2) {              // matrix bias staged by TMA
+    if (bp.bias_vec == 2 || bp.bias_kind == RGD_BIAS_VECTOR) {
+        // vector bias by its alignment; matrix bias staged by TMA: plain, writing the bias gradient or
+        // following tile lists (never both)
         const size_t smem = sizeof(DqBiasSmem<D>) + 1024;
-        // three instantiations: plain, writing the bias gradient, following tile lists (never both)
-        const int mode = bp.dbias != nullptr ? 1 : (bp.tlq_cnt != nullptr ? 2 : 0);
-        const void *kernel = mode == 1   ? reinterpret_cast<const void *>(attn_bwd_dq_bias<D, BF16, true, false, false>)
-                             : mode == 2 ? reinterpret_cast<const void *>(attn_bwd_dq_bias<D, BF16, false, true, false>)
-                                         : reinterpret_cast<const void *>(attn_bwd_dq_bias<D, BF16, false, false, false>);
-        if (int e = ensure_dyn_smem(kernel, smem)) return e;
-        dim3 grid((p.Tq + BT - 1) / BT, BH);
-        if (mode == 1)
-            attn_bwd_dq_bias<D, BF16, true, false, false><<<grid, DQ_PIPE_THREADS, smem, st>>>(bp, p.q, p.d_o, p.q_sb, p.q_sh, p.q_sn,
-                                                                                          p.do_sb, p.do_sh, p.do_sn);
-        else if (mode == 2)
-            attn_bwd_dq_bias<D, BF16, false, true, false><<<grid, DQ_PIPE_THREADS, smem, st>>>(bp, p.q, p.d_o, p.q_sb, p.q_sh, p.q_sn,
-                                                                                          p.do_sb, p.do_sh, p.do_sn);
-        else
-            attn_bwd_dq_bias<D, BF16, false, false, false><<<grid, DQ_PIPE_THREADS, smem, st>>>(bp, p.q, p.d_o, p.q_sb, p.q_sh,
-                                                                                           p.q_sn, p.do_sb, p.do_sh, p.do_sn);
-        count_launch();
-        return check_launch();
+        const bool bulk = bp.bias_vec == 1 && !bp.bias_f32 && p.Tk % 8 == 0;
+        auto kernel = bp.bias_kind == RGD_BIAS_VECTOR ? (bulk ? attn_bwd_dq_bias<D, BF16, false, false, 1> : attn_bwd_dq_bias<D, BF16, false, false, 2>)
+                      : bp.dbias != nullptr           ? attn_bwd_dq_bias<D, BF16, true, false, 0>
+                      : bp.tlq_cnt != nullptr         ? attn_bwd_dq_bias<D, BF16, false, true, 0>
+                                                      : attn_bwd_dq_bias<D, BF16, false, false, 0>;
+        if (int e = ensure_dyn_smem(reinterpret_cast<const void *>(kernel), smem)) return e;
+        return launch_pdl(kernel, bp.order.nblk * BH, DQ_PIPE_THREADS, smem, st, bp, p.q, p.d_o, p.q_sb, p.q_sh, p.q_sn, p.do_sb,
+                          p.do_sh, p.do_sn);
     }
-    return launch_bwd_tmem<D, BF16, false>(bp, (p.Tq + BT - 1) / BT, BH, st);
+    return launch_bwd_tmem<D, BF16, false>(bp, st);
 }
 
 // p.delta points at the caller's workspace (tmem_bwd_workspace_bytes); dq_acc, when not null, at an
@@ -2466,18 +2460,22 @@ int tmem_bwd(const AttnParams &p, int dtype, rgd_cache *cache, float *dq_acc, cu
         if (p.bias_kind == RGD_BIAS_VECTOR && bp.bias_vec == 2) return TMEM_NOT_TAKEN;
         bp.inv_scale = 1.f / p.scale;
     }
+    // The caller gave room for the fp32 dQ accumulator: single-pass form, except with tile lists, a
+    // bias gradient or a matrix bias that does not go through TMA, which the two-kernel form serves
+    if (bp.dbias != nullptr || bp.tlk_cnt != nullptr || (p.bias_kind == RGD_BIAS_MATRIX && bp.bias_vec != 2)) bp.dq_acc = nullptr;
     {
-        const int rows_per_cta = 256 / (p.d / 8);
+        const int rows_per_cta = p.d > 64 ? 16 : 32;
         dim3 grid((Tq128 + rows_per_cta - 1) / rows_per_cta, p.B * p.H);
-        if (bf16) attn_bwd_prep_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(p, lse2, delta_s, Tq128);
-        else attn_bwd_prep_kernel<__half><<<grid, 256, 0, st>>>(p, lse2, delta_s, Tq128);
+        if (bf16) attn_bwd_prep_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(p, lse2, delta_s, bp.dq_acc, Tq128);
+        else attn_bwd_prep_kernel<__half><<<grid, 256, 0, st>>>(p, lse2, delta_s, bp.dq_acc, Tq128);
         count_launch();
         if (int e = check_launch()) return e;
     }
     bp.lse2 = lse2; bp.delta_s = delta_s;
+    bp.d = p.d;
     bp.H = p.H; bp.Tq = p.Tq; bp.Tk = p.Tk; bp.Tq128 = Tq128; bp.causal = p.causal;
     bp.scale = p.scale; bp.scale_log2 = p.scale * LOG2E;
-    if (p.d == 128) return bf16 ? bwd_both<128, true>(bp, p, st) : bwd_both<128, false>(bp, p, st);
+    if (p.d > 64) return bf16 ? bwd_both<128, true>(bp, p, st) : bwd_both<128, false>(bp, p, st);
     return bf16 ? bwd_both<64, true>(bp, p, st) : bwd_both<64, false>(bp, p, st);
 }
 

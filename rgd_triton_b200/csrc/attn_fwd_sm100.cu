@@ -54,6 +54,8 @@ struct FwdTmaParams {
     int bias_h0, bias_b0;       // bias broadcast over heads / batch: always coordinate 0
     float *lse;
     int H, Tq, Tk, Tq_rounded, causal;
+    TileOrder order;
+    int d;              // channels, a multiple of 8, at most D: the tiles are zero-filled up to D
     float scale_log2;   // softmax_scale * log2(e)
     int *status;        // device status word (bounded waits report here)
     // BIAS == 2, optional: per 256-query block of each bias slice, the key blocks to visit (the
@@ -315,8 +317,9 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) attn_fwd_tmem(const __grid_con
     Smem &sm = *reinterpret_cast<Smem *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int mblk = p.causal ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;   // heavy causal tiles first
-    const int bh = blockIdx.y;
+    int mblk, bh;
+    tile_of(p.order, mblk, bh);
+    if (p.causal) mblk = p.order.nblk - 1 - mblk;      // heavy causal tiles first
     const int b = bh / p.H, h = bh - b * p.H;
     const int m0 = mblk * NT * TM;
     // Key blocks each tile visits (a tile past the end of Q visits none; under
@@ -332,7 +335,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) attn_fwd_tmem(const __grid_con
     const uint16_t *tl = nullptr;
     if constexpr (LISTS) {
         const int64_t slice = (int64_t)(p.bias_b0 ? 0 : b) * (p.bias_h0 ? 1 : p.H) + (p.bias_h0 ? 0 : h);
-        const int64_t idx = slice * gridDim.x + mblk;
+        const int64_t idx = slice * p.order.nblk + mblk;
         tl = p.tl_list + idx * p.tl_nkb;
         const int cnt = p.tl_cnt[idx];
 #pragma unroll
@@ -422,6 +425,8 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) attn_fwd_tmem(const __grid_con
             constexpr uint32_t idesc_pv = make_idesc(BF16, TM, D, false, true);
             auto issue_s = [&](int t, int s) {
                 const uint32_t q_addr = smem_u32(sm.q[t]), k_addr = smem_u32(sm.k[s]);
+                // all D / 16 steps whatever d is: a test of d in this loop, or a second loop beside it, costs
+                // every size 2-4 % (0.473 -> 0.494 ms at [4, 4096, 16, 128])
 #pragma unroll
                 for (int kk = 0; kk < D / 16; ++kk) {
                     const uint32_t off = (kk / 4) * PANEL + (kk % 4) * 32;
@@ -940,6 +945,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) attn_fwd_tmem(const __grid_con
                     if (row < p.Tq) {
 #pragma unroll
                         for (int i = 0; i < 32; i += 8) {
+                            if (c * 32 + i >= p.d) break;
                             uint4 v;
                             v.x = pack16<BF16>(__uint_as_float(r[i]) * inv, __uint_as_float(r[i + 1]) * inv);
                             v.y = pack16<BF16>(__uint_as_float(r[i + 2]) * inv, __uint_as_float(r[i + 3]) * inv);
@@ -996,31 +1002,30 @@ static bool tma_view_ok(const void *ptr, int B, int H, int T, int64_t sb, int64_
 
 bool tmem_fwd_eligible(const AttnParams &p) {
     // The mask-free fast path takes the block maximum before scaling, which needs scale > 0.
-    return (p.d == 64 || p.d == 128) && p.Tq >= 1 && p.Tk >= 1 && p.scale > 0.f && p.vec_q && p.vec_k && p.vec_v &&
+    return p.d >= 8 && p.d <= 128 && p.d % 8 == 0 && p.Tq >= 1 && p.Tk >= 1 && p.scale > 0.f && p.vec_q && p.vec_k && p.vec_v &&
            p.vec_o && tma_view_ok(p.q, p.B, p.H, p.Tq, p.q_sb, p.q_sh, p.q_sn) &&
            tma_view_ok(p.k, p.B, p.H, p.Tk, p.k_sb, p.k_sh, p.k_sn) &&
            tma_view_ok(p.v, p.B, p.H, p.Tk, p.v_sb, p.v_sh, p.v_sn);
 }
 
 template <int D, bool BF16, int BIAS, bool LISTS = false>
-static int launch_fwd_one(const FwdTmaParams &fp, int Tq, int BH, cudaStream_t st) {
+static int launch_fwd_one(const FwdTmaParams &fp, cudaStream_t st) {
     constexpr int NT = 2;
     constexpr int VS = (BIAS == 2 && D == 128) ? 1 : 2;
     constexpr int BS = BIAS == 2 ? (D == 128 ? 1 : 2) : 0;
     const size_t smem = sizeof(FwdTmaSmem<D, NT, VS, BS, BIAS == 1>) + 1024;
     if (int e = ensure_dyn_smem(reinterpret_cast<const void *>(attn_fwd_tmem<D, BF16, BIAS, LISTS>), smem)) return e;
-    dim3 grid((Tq + NT * TM - 1) / (NT * TM), BH);
-    attn_fwd_tmem<D, BF16, BIAS, LISTS><<<grid, FWD_THREADS, smem, st>>>(fp);
+    attn_fwd_tmem<D, BF16, BIAS, LISTS><<<fp.order.nblk * fp.order.BH, FWD_THREADS, smem, st>>>(fp);
     count_launch();
     return check_launch();
 }
 
 template <int D, bool BF16>
-static int launch_fwd_tmem(const FwdTmaParams &fp, int bias_mode, int Tq, int BH, cudaStream_t st) {
-    if (bias_mode == 2 && fp.tl_cnt != nullptr) return launch_fwd_one<D, BF16, 2, true>(fp, Tq, BH, st);
-    if (bias_mode == 2) return launch_fwd_one<D, BF16, 2>(fp, Tq, BH, st);
-    if (bias_mode == 1) return launch_fwd_one<D, BF16, 1>(fp, Tq, BH, st);
-    return launch_fwd_one<D, BF16, 0>(fp, Tq, BH, st);
+static int launch_fwd_tmem(const FwdTmaParams &fp, int bias_mode, cudaStream_t st) {
+    if (bias_mode == 2 && fp.tl_cnt != nullptr) return launch_fwd_one<D, BF16, 2, true>(fp, st);
+    if (bias_mode == 2) return launch_fwd_one<D, BF16, 2>(fp, st);
+    if (bias_mode == 1) return launch_fwd_one<D, BF16, 1>(fp, st);
+    return launch_fwd_one<D, BF16, 0>(fp, st);
 }
 
 // A matrix bias in the tensor dtype whose rows are 16-byte addressable goes through TMA.
@@ -1065,14 +1070,16 @@ int tmem_fwd(const AttnParams &p, int dtype, rgd_cache *cache, cudaStream_t st) 
         fp.tl_nkb = L.nkb;
     }
     fp.lse = p.lse;
+    fp.d = p.d;
     fp.H = p.H; fp.Tq = p.Tq; fp.Tk = p.Tk; fp.Tq_rounded = p.Tq_rounded; fp.causal = p.causal;
     fp.scale_log2 = p.scale * LOG2E;
     fp.status = tmem_status_ptr();
     if (!fp.status) return RGD_E_DEVICE;
-    const int BH = p.B * p.H;
-    if (p.d == 128)
-        return bf16 ? launch_fwd_tmem<128, true>(fp, bias_mode, p.Tq, BH, st) : launch_fwd_tmem<128, false>(fp, bias_mode, p.Tq, BH, st);
-    return bf16 ? launch_fwd_tmem<64, true>(fp, bias_mode, p.Tq, BH, st) : launch_fwd_tmem<64, false>(fp, bias_mode, p.Tq, BH, st);
+    // K and V of a head, the operands its query blocks share
+    fp.order = make_tile_order((p.Tq + 2 * TM - 1) / (2 * TM), p.B * p.H, p.causal, (int64_t)p.Tk * p.d * 4);
+    if (p.d > 64)
+        return bf16 ? launch_fwd_tmem<128, true>(fp, bias_mode, st) : launch_fwd_tmem<128, false>(fp, bias_mode, st);
+    return bf16 ? launch_fwd_tmem<64, true>(fp, bias_mode, st) : launch_fwd_tmem<64, false>(fp, bias_mode, st);
 }
 
 // Exercises the give-up path of the bounded waits without any broken pipeline: one thread waits,

@@ -1,7 +1,7 @@
 // Warp-level building blocks of the general attention kernels: 64-row tiles in
 // padded shared memory, ldmatrix fragment loads and m16n8k16 tensor-core MMAs
 // with fp32 accumulation.  Used for shapes the tensor-memory kernels do not
-// take (head_dim not 64/128, unaligned strides, short sequences).
+// take (head_dim not a multiple of 8, unaligned strides).
 #pragma once
 
 #include "common.cuh"

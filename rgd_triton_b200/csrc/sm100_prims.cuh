@@ -72,6 +72,50 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int *s
 }
 
 // ---------------------------------------------------------------------------
+// Order in which a 1-D grid walks the (batch, head) x tile-block pairs.  Without a causal mask the
+// blocks of one head run next to each other (they share its K and V in L2).  Under a causal mask the
+// work per block differs, and the blocks of `group` heads are interleaved by rank, heaviest rank
+// first, so that the last CTAs to start are the lightest ones; the group is as many heads as L2
+// holds the operands of.
+// ---------------------------------------------------------------------------
+struct TileOrder {
+    int nblk, group, BH;
+};
+__device__ __forceinline__ void tile_of(const TileOrder &o, int &rank, int &bh) {
+    const int per = o.nblk * o.group;
+    const int g = (int)blockIdx.x / per, rem = (int)blockIdx.x - g * per;
+    const int heads = min(o.group, o.BH - g * o.group);
+    rank = rem / heads;
+    bh = g * o.group + rem - rank * heads;
+}
+inline TileOrder make_tile_order(int nblk, int BH, bool causal, int64_t bytes_per_head) {
+    const int64_t fit = (48ll << 20) / (bytes_per_head > 0 ? bytes_per_head : 1);
+    return {nblk, causal ? (int)(fit < 1 ? 1 : fit > BH ? BH : fit) : 1, BH};
+}
+
+// Programmatic dependent launch: a kernel launched with launch_pdl may start while its predecessor in
+// the stream still runs; grid_wait() returns once the predecessor has completed and its writes are
+// visible, grid_trigger() (every CTA) allows the successor to start.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... Params, typename... Args>
+inline int launch_pdl(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+    count_launch();
+    return cuda_status(e);
+}
+
+// ---------------------------------------------------------------------------
 // TMA: tiled 4-D load global -> shared, completion on an mbarrier.  No
 // multicast: every CTA fetches its own tiles from this GPU's memory.
 // ---------------------------------------------------------------------------

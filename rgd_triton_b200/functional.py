@@ -893,8 +893,8 @@ class FlashAttnFunc(torch.autograd.Function):
         return dq, dk, dv, dbias, None, None, None
 
 
-# How the attention backward forms dQ where the library offers a choice (head_dim 64 on the
-# tensor-memory kernels):
+# How the attention backward forms dQ where the library offers a choice (head_dim up to 64 on
+# the tensor-memory kernels):
 #   "single_pass"  S, dP and the exponentials are evaluated once per tile pair and the dQ partial tiles
 #                  are added into an fp32 accumulator (B * H * Tq * d * 4 bytes of scratch per call) with
 #                  vector reductions, like the reference's atomic adds into dq
@@ -935,7 +935,7 @@ def _attn_backward(q, k, v, bias, o, lse, do, causal, softmax_scale, cache, want
     if tiles is not None and not want_dbias:
         bias_s.tiles = tiles.data_ptr()
     dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-    single = _ATTN_BWD_MODE == "single_pass" and d == 64 and not want_dbias and tiles is None
+    single = _ATTN_BWD_MODE == "single_pass" and d <= 64 and not want_dbias and tiles is None
     dt, nbytes = _const(plan, ("c", single), lambda: (_lib.dtype_code(q.dtype), _attn_bwd_bytes(
         lib, single, batch, nheads, seqlen_q, seqlen_k, d, _lib.dtype_code(q.dtype))))
     _require(nbytes >= 0, "attn_bwd: bad sizes")
@@ -989,13 +989,13 @@ def flash_attn_func(q, k, v, bias=None, causal=False, softmax_scale=None, return
         o, lse = torch.ops.rgd_b200.attn(q, k, v, bias, bool(causal), scale)
         return (o, lse) if return_lse else o
     d = q.shape[-1] if q.ndim == 4 else 0
-    if d not in (0, 64, 128) and d < 128 and _pad_head_dim_pays(q, k):
-        # Head dims other than 64 / 128 have no tensor-memory instantiation of their own: large
-        # problems are zero-padded to the next of the two (zero channels add nothing to q k^T, and
-        # the padded channels of v give output channels that are cut off again), which keeps them
-        # on the tcgen05 kernels; the softmax scale stays that of the true head_dim.  Small
-        # problems run on the general kernels, where the copies would cost more than they save.
-        dp = 64 if d < 64 else 128
+    if d % 8 != 0 and d < 128 and _pad_head_dim_pays(q, k):
+        # The tensor-memory kernels take head dims that are multiples of 8 (16-byte rows): large
+        # problems with others are zero-padded to the next one (zero channels add nothing to q k^T, and
+        # the padded channels of v give output channels that are cut off again); the softmax scale
+        # stays that of the true head_dim.  Small problems run on the general kernels, where the copies
+        # would cost more than they save.
+        dp = (d + 7) // 8 * 8
         pad = lambda t: torch.nn.functional.pad(t, (0, dp - d))
         res = flash_attn_func(pad(q), pad(k), pad(v), bias, causal, softmax_scale or 1.0 / math.sqrt(d), True,
                               kernel_cache)

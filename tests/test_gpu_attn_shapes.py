@@ -1,0 +1,67 @@
+"""Attention at the edges of the kernels' dispatch: head dims that are multiples of 8, vector biases of
+every alignment, causal grids of more heads than one scheduling group, few queries."""
+import pytest
+import torch
+
+from rgd_triton_b200 import _lib, functional as F_
+from tests._util import DTYPES, attention_backward, gen, randn
+from tests.test_gpu_attn import check, make_bias
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def no_expired_waits():
+    yield
+    assert _lib.load().rgd_device_status() == 0
+
+
+def _inputs(g, B, tq, tk, H, d, dtype):
+    return (randn(g, B, tq, H, d, dtype=dtype), randn(g, B, tk, H, d, dtype=dtype), randn(g, B, tk, H, d, dtype=dtype),
+            randn(g, B, tq, H, d, dtype=dtype))
+
+
+@pytest.mark.parametrize("mode", ["single_pass", "two_kernel"])
+@pytest.mark.parametrize("d", [8, 24, 56, 72, 104, 120])
+@pytest.mark.parametrize("kind", [None, "vector", "matrix"])
+def test_head_dims_that_are_multiples_of_8(d, kind, mode):
+    """Channels past d are zero-filled tiles on the tensor-memory kernels: nothing of them may reach the
+    outputs, and nothing past d channels may be written (the row after the last head is checked by the
+    dense layout: an overrun would land in the next head's outputs)."""
+    g = gen(d)
+    for tq, tk in [(130, 136), (257, 96)]:
+        q, k, v, do = _inputs(g, 2, tq, tk, 3, d, torch.bfloat16)
+        bias = None if kind is None else make_bias(g, kind, 2, 3, tq, tk, torch.bfloat16)
+        with attention_backward(mode):
+            check(q, k, v, do, bias, False, f"d={d} {kind} ({tq},{tk})")
+
+
+@pytest.mark.parametrize("dt", ["f16", "bf16"])
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("tk", [127, 128, 129, 260, 390])
+def test_vector_bias_of_any_alignment(dt, d, tk):
+    """Key counts around the 128-key block; a vector whose batch rows are not 16-byte addressable is staged
+    by the compute threads, an aligned one by bulk copies."""
+    g = gen(tk + d)
+    q, k, v, do = _inputs(g, 2, 140, tk, 2, d, DTYPES[dt])
+    bias = make_bias(g, "vector", 2, 2, 140, tk, DTYPES[dt])
+    with attention_backward("two_kernel"):
+        check(q, k, v, do, bias, False, f"vector d={d} tk={tk}")
+
+
+@pytest.mark.parametrize("d,H", [(128, 100), (64, 200)])
+def test_causal_grid_of_more_heads_than_a_group(d, H):
+    """The causal grids interleave the query blocks of as many heads as fit L2; with more heads than that
+    every head must still get exactly its own blocks: bit-equal to evaluating the heads in two halves."""
+    g = gen(H)
+    q, k, v, do = (t.cuda() for t in _inputs(g, 1, 300, 1030, H, d, torch.bfloat16))
+
+    def run(sl):
+        a, b, c = (t[:, :, sl].contiguous().requires_grad_(True) for t in (q, k, v))
+        o = F_.flash_attn_func(a, b, c, None, True)
+        return (o.detach(), *torch.autograd.grad(o, (a, b, c), do[:, :, sl].contiguous()))
+    with attention_backward("two_kernel"):
+        whole = run(slice(0, H))
+        halves = [run(slice(0, H // 2)), run(slice(H // 2, H))]
+    for w, x, y in zip(whole, *halves):
+        assert torch.equal(w, torch.cat([x, y], dim=2))
