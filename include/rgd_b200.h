@@ -332,8 +332,9 @@ int rgd_attn_bwd_dbias(const rgd_heads *q, const rgd_heads *k,
                        rgd_cache *cache, void *stream);
 
 /* Which attention implementation rgd_attn_fwd / rgd_attn_bwd take for these
- * views: 1 = tcgen05 / tensor-memory / TMA kernels, 0 = general mma.sync
- * kernels.  Evaluates exactly the test the entry points use (head_dim a
+ * views: 1 = tcgen05 / tensor-memory / TMA kernels, 0 = mma.sync kernels (the
+ * general ones, and the forward for at most 16 queries without a causal mask).
+ * Evaluates exactly the test the entry points use (head_dim a
  * multiple of 8, every view 16-byte addressable with positive strides on dimensions of
  * extent > 1, and for the forward softmax_scale > 0). */
 int rgd_attn_fwd_uses_tmem(const rgd_heads *q, const rgd_heads *k,

@@ -10,6 +10,8 @@ int general_bwd(const AttnParams &p, int dtype, cudaStream_t st);
 bool tmem_fwd_eligible(const AttnParams &p);
 int tmem_fwd(const AttnParams &p, int dtype, rgd_cache *cache, cudaStream_t st);
 int tmem_status_fetch();
+bool few_fwd_eligible(const AttnParams &p);
+int few_fwd(const AttnParams &p, int dtype, cudaStream_t st);
 bool tmem_bwd_eligible(const AttnParams &p);
 int tmem_bwd(const AttnParams &p, int dtype, rgd_cache *cache, float *dq_acc, cudaStream_t st);
 int64_t single_pass_acc_offset(int64_t B, int64_t H, int64_t Tq);
@@ -123,6 +125,8 @@ extern "C" int rgd_attn_fwd(const rgd_heads *q, const rgd_heads *k, const rgd_he
     AttnParams p{};
     fill_fwd(p, q, k, v, bias, o, B, H, Tq, Tk, d, softmax_scale, causal);
     p.lse = lse;
+    // at most 16 queries: the chip is bound by reading K and V once, which the split-key kernel is built for
+    if (work && attn::few_fwd_eligible(p)) return attn::few_fwd(p, dtype, (cudaStream_t)stream);
     if (work && attn::tmem_fwd_eligible(p)) {
         const int rc = attn::tmem_fwd(p, dtype, cache, (cudaStream_t)stream);
         if (rc != attn::TMEM_NOT_TAKEN) return rc;
@@ -136,7 +140,7 @@ extern "C" int rgd_attn_fwd_uses_tmem(const rgd_heads *q, const rgd_heads *k, co
     if (check_common(q, k, v, nullptr, B, H, Tq, Tk, d, dtype) != RGD_OK || !o) return 0;
     AttnParams p{};
     fill_fwd(p, q, k, v, nullptr, o, B, H, Tq, Tk, d, softmax_scale, 0);
-    return (B > 0 && H > 0 && Tq > 0 && attn::tmem_fwd_eligible(p)) ? 1 : 0;
+    return (B > 0 && H > 0 && Tq > 0 && !attn::few_fwd_eligible(p) && attn::tmem_fwd_eligible(p)) ? 1 : 0;
 }
 
 extern "C" int64_t rgd_attn_bwd_workspace_bytes(int64_t B, int64_t H, int64_t Tq, int64_t Tk, int64_t d, int dtype) {

@@ -65,3 +65,33 @@ def test_causal_grid_of_more_heads_than_a_group(d, H):
         halves = [run(slice(0, H // 2)), run(slice(H // 2, H))]
     for w, x, y in zip(whole, *halves):
         assert torch.equal(w, torch.cat([x, y], dim=2))
+
+
+@pytest.mark.parametrize("dt", ["f16", "bf16"])
+@pytest.mark.parametrize("d", [8, 40, 64, 96, 128])
+@pytest.mark.parametrize("kind", [None, "vector", "matrix", "matrix_f32"])
+def test_few_queries(dt, d, kind):
+    """At most 16 queries: the split-key kernel.  Query counts around its 8-row halves, key counts around its
+    16-key tiles and from one tile (one CTA) to enough for every cluster size."""
+    dtype = DTYPES[dt]
+    g = gen(d)
+    for tq, tk in [(1, 1), (1, 15), (2, 16), (8, 17), (9, 64), (16, 129), (3, 1000), (16, 2100)]:
+        q, k, v, do = _inputs(g, 2, tq, tk, 3, d, dtype)
+        bias = None if kind is None else make_bias(g, kind, 2, 3, tq, tk, dtype)
+        check(q, k, v, do, bias, False, f"few d={d} {kind} ({tq},{tk})")
+
+
+def test_few_queries_many_heads_and_masked_keys():
+    """More heads than CTAs the chip holds (other split), K / V expanded over the batch (stride 0), a fully
+    masked first half of the keys (a warp whose tiles are all masked contributes nothing)."""
+    g = gen(5)
+    B, H, tk, d = 5, 70, 300, 64
+    q = randn(g, B, 4, H, d, dtype=torch.float16).cuda()
+    k, v = (randn(g, 1, tk, H, d, dtype=torch.float16).cuda().expand(B, tk, H, d) for _ in range(2))
+    bias = torch.zeros(B, 1, 1, tk, dtype=torch.float16)
+    bias[..., :150] = float("-inf")
+    got = F_.flash_attn_func(q, k, v, bias.cuda())
+    s = torch.einsum("bqhd,bkhd->bhqk", q.float(), k.float()) / d ** 0.5 + bias.cuda().float()
+    want = torch.einsum("bhqk,bkhd->bqhd", s.softmax(-1), v.float())
+    # P and the output are rounded to fp16: two half-ulp roundings of values of magnitude < 4
+    assert (got.float() - want).abs().max().item() < 4 * 2 ** -10
