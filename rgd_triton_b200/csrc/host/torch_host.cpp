@@ -7,7 +7,7 @@
 // autograd.Function, launch keys built from Python tuples) such a call took 126 us, a forward alone 15 us.
 //
 // Every entry returns None for arguments it does not cover: anything that is wrong (the Python path then
-// raises the right exception), tensor subclasses, views whose channel stride is not 1, empty tensors,
+// raises the right exception), tensor subclasses, forward-mode tangents, views whose channel stride is not 1, empty tensors,
 // caches that are not a _LaunchCache, a bias that wants a gradient.  The Python path in functional.py
 // handles those, so conditions here only have to be sufficient.
 //
@@ -86,10 +86,13 @@ int code_of(const Tensor &t) {
     }
 }
 
+// A tensor that only Python knows how to handle, or that carries a forward-mode tangent (the autograd
+// functions have no jvp: the Python path refuses it).
+bool special(const Tensor &t) { return t.unsafeGetTensorImpl()->is_python_dispatch() || t._fw_grad(0).defined(); }
+
 // A plain CUDA tensor of a supported type with unit channel stride and at least one element.
 bool plain(const Tensor &t, int64_t ndim) {
-    return t.defined() && t.is_cuda() && t.dim() == ndim && t.numel() > 0 && t.stride(-1) == 1 && code_of(t) >= 0 &&
-           !t.unsafeGetTensorImpl()->is_python_dispatch();
+    return t.defined() && t.is_cuda() && t.dim() == ndim && t.numel() > 0 && t.stride(-1) == 1 && code_of(t) >= 0 && !special(t);
 }
 
 bool like(const Tensor &t, const Tensor &first) {
@@ -208,6 +211,15 @@ PyObject *wrap2(Tensor a, Tensor b) {
     return t;
 }
 
+// Allocation and launches run without the GIL, as they do through ctypes: a full launch queue or a
+// first allocation then stops no other Python thread.
+struct NoGil {
+    PyThreadState *saved = PyEval_SaveThread();
+    NoGil() = default;
+    NoGil(const NoGil &) = delete;
+    ~NoGil() { PyEval_RestoreThread(saved); }
+};
+
 // ------------------------------------------------------------------ row norms
 rgd_rows rows(const Tensor &t) { return {t.data_ptr(), t.stride(0), t.stride(1)}; }
 
@@ -236,7 +248,7 @@ bool rows_ok(Rows &r) {
         const Tensor &w = r.w[i];
         if (!w.defined()) continue;
         if (!w.is_cuda() || w.device() != a.device() || code_of(w) < 0 || w.scalar_type() != r.w[0].scalar_type() ||
-            w.unsafeGetTensorImpl()->is_python_dispatch() || (w.dim() != 1 && w.dim() != 3) || w.stride(-1) != 1 ||
+            special(w) || (w.dim() != 1 && w.dim() != 3) || w.stride(-1) != 1 ||
             w.size(-1) != r.C[i])
             return false;
         if (w.dim() == 3) {
@@ -252,6 +264,7 @@ bool rows_ok(Rows &r) {
 }
 
 void rows_forward(Rows &r, Tensor (&y)[2]) {
+    NoGil nogil;
     c10::cuda::OptionalCUDAGuard guard(r.x[0].device());
     rgd_rows xs[2], ys[2];
     const void *ws[2] = {nullptr, nullptr};
@@ -474,10 +487,15 @@ struct HeadsBackward : public Node {
 };
 
 PyObject *heads_call(Heads &h, const Tensor &q, const Tensor &k, const Tensor &pos) {
-    c10::cuda::OptionalCUDAGuard guard(q.device());
-    Tensor qo = new_like(q), ko = new_like(k);
-    heads_launch(h, false, q, k, Tensor(), Tensor(), pos, qo, ko);
-    note(h.state, 0, q, k);
+    Tensor qo, ko;
+    {
+        NoGil nogil;
+        c10::cuda::OptionalCUDAGuard guard(q.device());
+        qo = new_like(q);
+        ko = new_like(k);
+        heads_launch(h, false, q, k, Tensor(), Tensor(), pos, qo, ko);
+        note(h.state, 0, q, k);
+    }
     if (wants_grad({&q, &k})) {
         auto node = new_node<HeadsBackward>(torch::autograd::collect_next_edges(q, k));
         node->h = h;
@@ -572,14 +590,18 @@ struct AttnBackward : public Node {
 
 PyObject *attn_call(Attn &a, const Tensor &q, const Tensor &k, const Tensor &v, const Tensor &bias, const Tensor &tiles,
                     bool return_lse) {
-    c10::cuda::OptionalCUDAGuard guard(q.device());
-    Tensor o = new_like(q);
-    Tensor lse = new_buffer({a.B, a.H, api.attn_lse_rows(a.tq)}, at::kFloat, q.device());
-    const rgd_heads qv = Attn::view(q), kv = Attn::view(k), vv = Attn::view(v), ov = Attn::view(o);
-    const rgd_bias b = a.bias(bias, tiles);
-    launched(api.attn_fwd(&qv, &kv, &vv, &b, &ov, lse.data_ptr<float>(), a.B, a.H, a.tq, a.tk, a.d, (float)a.scale,
-                          a.causal ? 1 : 0, a.dtype, a.state ? a.state->native() : nullptr, stream_of(q)), "attn_fwd", true);
-    note(a.state, 0, q, k, v);
+    Tensor o, lse;
+    {
+        NoGil nogil;
+        c10::cuda::OptionalCUDAGuard guard(q.device());
+        o = new_like(q);
+        lse = new_buffer({a.B, a.H, api.attn_lse_rows(a.tq)}, at::kFloat, q.device());
+        const rgd_heads qv = Attn::view(q), kv = Attn::view(k), vv = Attn::view(v), ov = Attn::view(o);
+        const rgd_bias b = a.bias(bias, tiles);
+        launched(api.attn_fwd(&qv, &kv, &vv, &b, &ov, lse.data_ptr<float>(), a.B, a.H, a.tq, a.tk, a.d, (float)a.scale,
+                              a.causal ? 1 : 0, a.dtype, a.state ? a.state->native() : nullptr, stream_of(q)), "attn_fwd", true);
+        note(a.state, 0, q, k, v);
+    }
     if (wants_grad({&q, &k, &v})) {
         auto node = new_node<AttnBackward>(torch::autograd::collect_next_edges(q, k, v));
         node->a = a;
