@@ -2296,7 +2296,10 @@ __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __grid_constan
     if (l == 0 && i < Tq128) {
         const int64_t idx = (int64_t)bh * Tq128 + i;
         delta_s[idx] = a * p.scale;
-        lse2[idx] = i < p.Tq ? p.lse[(int64_t)bh * p.Tq_rounded + i] * LOG2E : INFINITY;
+        // A row whose keys are all masked with a huge value (or -inf) has no P that lse still resolves
+        // (2^(x - lse2) would be inf or 0 by rounding): it passes no gradient on, like a row past the end.
+        const float lse = i < p.Tq ? p.lse[(int64_t)bh * p.Tq_rounded + i] : INFINITY;
+        lse2[idx] = lse < -1e7f ? INFINITY : lse * LOG2E;
     }
 }
 

@@ -100,7 +100,7 @@ __device__ __forceinline__ void bias_from_smem(const unsigned char *tile, int ro
         union { uint4 u; T v[8]; } cv;
         cv.u = *reinterpret_cast<const uint4 *>(rowp + (((c0 + i) ^ (row_l & 7)) << 4));
 #pragma unroll
-        for (int e = 0; e < 8; ++e) b[8 * i + e] = to_f32<T>(cv.v[e]) * LOG2E;
+        for (int e = 0; e < 8; ++e) b[8 * i + e] = BF16 ? bias_log2(to_f32<T>(cv.v[e])) : to_f32<T>(cv.v[e]) * LOG2E;
     }
 }
 
@@ -133,11 +133,11 @@ __device__ __forceinline__ void load_bias32(const FwdTmaParams &p, const char *b
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const float4 v = reinterpret_cast<const float4 *>(src)[i];
-                b[4 * i] = v.x * LOG2E; b[4 * i + 1] = v.y * LOG2E; b[4 * i + 2] = v.z * LOG2E; b[4 * i + 3] = v.w * LOG2E;
+                b[4 * i] = bias_log2(v.x); b[4 * i + 1] = bias_log2(v.y); b[4 * i + 2] = bias_log2(v.z); b[4 * i + 3] = bias_log2(v.w);
             }
         } else {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) b[i] = (col0 + i < p.Tk) ? src[i] * LOG2E : 0.f;
+            for (int i = 0; i < 32; ++i) b[i] = (col0 + i < p.Tk) ? bias_log2(src[i]) : 0.f;
         }
     } else {
         const T *src = reinterpret_cast<const T *>(bias_bh) + off;
@@ -146,11 +146,11 @@ __device__ __forceinline__ void load_bias32(const FwdTmaParams &p, const char *b
             for (int i = 0; i < 4; ++i) {
                 const Vec<T, 8> v = load_vec<T, 8>(src + 8 * i);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) b[8 * i + e] = to_f32<T>(v.v[e]) * LOG2E;
+                for (int e = 0; e < 8; ++e) b[8 * i + e] = bias_log2(to_f32<T>(v.v[e]));
             }
         } else {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) b[i] = (col0 + i < p.Tk) ? to_f32<T>(src[i]) * LOG2E : 0.f;
+            for (int i = 0; i < 32; ++i) b[i] = (col0 + i < p.Tk) ? bias_log2(to_f32<T>(src[i])) : 0.f;
         }
     }
 }
@@ -519,7 +519,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) attn_fwd_tmem(const __grid_con
                     if (kj < p.Tk)
                         bvl = p.bias_f32 ? reinterpret_cast<const float *>(bias_bh)[kj]
                                          : to_f32<T>(reinterpret_cast<const T *>(bias_bh)[kj]);
-                    sm.vbias[t][j & 1][row_l] = bvl * LOG2E;
+                    sm.vbias[t][j & 1][row_l] = bias_log2(bvl);
                     mbar_arrive(&sm.vb_ready[t]);
                 }
             }

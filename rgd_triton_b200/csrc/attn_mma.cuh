@@ -14,6 +14,10 @@ constexpr int BN = 64;          // key rows per tile
 constexpr int NTHREADS = 128;   // 4 warps, 16 tile rows each
 constexpr int PAD = 8;          // 16-byte row padding: conflict-free ldmatrix
 constexpr float LOG2E = 1.4426950408889634f;
+
+// bias * log2(e), rounded towards zero: a mask near the lowest fp32 / bf16 value stays finite, so that a row
+// whose keys are all masked with it is uniform and not empty; -inf stays -inf.
+__device__ __forceinline__ float bias_log2(float b) { return __fmul_rz(b, LOG2E); }
 // Internal answer of the tensor-memory entry points: nothing was launched, run the general kernels.
 constexpr int TMEM_NOT_TAKEN = -1000;
 

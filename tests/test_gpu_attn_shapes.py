@@ -95,3 +95,29 @@ def test_few_queries_many_heads_and_masked_keys():
     want = torch.einsum("bhqk,bkhd->bqhd", s.softmax(-1), v.float())
     # P and the output are rounded to fp16: two half-ulp roundings of values of magnitude < 4
     assert (got.float() - want).abs().max().item() < 4 * 2 ** -10
+
+
+@pytest.mark.parametrize("d", [40, 64, 96, 128])
+@pytest.mark.parametrize("tq,tk", [(5, 40), (130, 200)])
+@pytest.mark.parametrize("kind", ["vector", "matrix", "matrix_f32"])
+def test_rows_masked_with_the_lowest_value(d, tq, tk, kind):
+    """One sequence masked by the type's lowest value in every key (its product with log2(e) overflows fp32):
+    its output is the mean of V, its gradients finite; the other sequence is as without a mask."""
+    g = gen(d + tq)
+    q, k, v, do = (t.cuda() for t in _inputs(g, 2, tq, tk, 3, d, torch.bfloat16))
+    dt = torch.float32 if kind == "matrix_f32" else torch.bfloat16
+    bias = torch.zeros(2, 1, 1 if kind == "vector" else tq, tk, dtype=dt, device="cuda")
+    bias[1] = torch.finfo(dt).min
+
+    def run(b):
+        leaves = [t.clone().requires_grad_(True) for t in (q, k, v)]
+        o = F_.flash_attn_func(*leaves, b)
+        return [o.detach(), *torch.autograd.grad(o, leaves, do)]
+    got, plain = run(bias), run(None)
+    want = v[1].float().mean(0, keepdim=True).expand(tq, -1, -1)
+    # P (1 here) is exact, the output is rounded to bf16: half an ulp of values below 2
+    assert (got[0][1].float() - want).abs().max().item() < 2.0 ** -8
+    for a, b in zip(got, plain):
+        assert torch.isfinite(a).all()
+        # two kernels' roundings of P and dS to bf16, summed over up to 200 keys or queries
+        assert (a[0].float() - b[0].float()).norm() <= 1e-2 * b[0].float().norm()
