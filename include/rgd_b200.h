@@ -334,9 +334,11 @@ int rgd_attn_bwd_dbias(const rgd_heads *q, const rgd_heads *k,
 /* Which attention implementation rgd_attn_fwd / rgd_attn_bwd take for these
  * views: 1 = tcgen05 / tensor-memory / TMA kernels, 0 = mma.sync kernels (the
  * general ones, and the forward for at most 16 queries without a causal mask).
- * Evaluates exactly the test the entry points use (head_dim a
+ * Evaluates the test the entry points use without a bias (head_dim a
  * multiple of 8, every view 16-byte addressable with positive strides on dimensions of
- * extent > 1, and for the forward softmax_scale > 0). */
+ * extent > 1, and for the forward softmax_scale > 0).  Below 2^24 scores a matrix bias that is
+ * fp32 or has rows that are not 16-byte addressable keeps head dims other than 64 / 128 on the
+ * general kernels. */
 int rgd_attn_fwd_uses_tmem(const rgd_heads *q, const rgd_heads *k,
                            const rgd_heads *v, const rgd_heads *o, int64_t B,
                            int64_t H, int64_t Tq, int64_t Tk, int64_t d,

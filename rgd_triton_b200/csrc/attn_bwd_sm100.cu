@@ -33,6 +33,7 @@ using namespace rgd::sm100;
 
 int *tmem_status_ptr();   // attn_fwd_sm100.cu
 bool bias_tma_ok(const AttnParams &p);
+bool general_takes_bias(const AttnParams &p);
 int encode_bias_map(rgd_cache *cache, CUtensorMap *out, const AttnParams &p, bool bf16, int box_q);
 
 constexpr int BWD_THREADS = 320;
@@ -2323,7 +2324,7 @@ int64_t single_pass_acc_bytes(int64_t B, int64_t H, int64_t Tq, int64_t d) {
 }
 
 bool tmem_bwd_eligible(const AttnParams &p) {
-    return p.d >= 8 && p.d <= 128 && p.d % 8 == 0 && p.Tq >= 1 && p.Tk >= 1 && p.vec_q && p.vec_k && p.vec_v && p.vec_o && p.vec_do &&
+    return !general_takes_bias(p) && p.d >= 8 && p.d <= 128 && p.d % 8 == 0 && p.Tq >= 1 && p.Tk >= 1 && p.vec_q && p.vec_k && p.vec_v && p.vec_o && p.vec_do &&
            p.vec_dq && p.vec_dk && p.vec_dv && heads_map_encodable(p.q, p.B, p.H, p.Tq, p.q_sb, p.q_sh, p.q_sn) &&
            heads_map_encodable(p.k, p.B, p.H, p.Tk, p.k_sb, p.k_sh, p.k_sn) &&
            heads_map_encodable(p.v, p.B, p.H, p.Tk, p.v_sb, p.v_sh, p.v_sn) &&

@@ -1000,9 +1000,19 @@ static bool tma_view_ok(const void *ptr, int B, int H, int T, int64_t sb, int64_
     return heads_map_encodable(ptr, B, H, T, sb, sh, sn);
 }
 
+bool bias_tma_ok(const AttnParams &p);
+// A matrix bias that TMA cannot stage (fp32, unaligned rows) is read by the threads, element by element in the
+// masked blocks.  At head dims 64 and 128 and in large problems that still beats the general kernels; in small
+// ones of other head dims it does not (forward [2, 324, 1, 32] bf16: 44 us here, 32 there).  The line is
+// that of the zero-padding on the host side.
+bool general_takes_bias(const AttnParams &p) {
+    return p.bias_kind == RGD_BIAS_MATRIX && !bias_tma_ok(p) && p.d != 64 && p.d != 128 &&
+           (int64_t)p.B * p.H * p.Tq * p.Tk < (int64_t)1 << 24;
+}
+
 bool tmem_fwd_eligible(const AttnParams &p) {
     // The mask-free fast path takes the block maximum before scaling, which needs scale > 0.
-    return p.d >= 8 && p.d <= 128 && p.d % 8 == 0 && p.Tq >= 1 && p.Tk >= 1 && p.scale > 0.f && p.vec_q && p.vec_k && p.vec_v &&
+    return !general_takes_bias(p) && p.d >= 8 && p.d <= 128 && p.d % 8 == 0 && p.Tq >= 1 && p.Tk >= 1 && p.scale > 0.f && p.vec_q && p.vec_k && p.vec_v &&
            p.vec_o && tma_view_ok(p.q, p.B, p.H, p.Tq, p.q_sb, p.q_sh, p.q_sn) &&
            tma_view_ok(p.k, p.B, p.H, p.Tk, p.k_sb, p.k_sh, p.k_sn) &&
            tma_view_ok(p.v, p.B, p.H, p.Tk, p.v_sb, p.v_sh, p.v_sn);
