@@ -28,6 +28,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -618,13 +619,17 @@ PyObject *attn_call(Attn &a, const Tensor &q, const Tensor &k, const Tensor &v, 
 }
 
 // ------------------------------------------------------------------ Python entries
-// C++ exceptions become Python ones; an argument the library refuses hands the call back (None).
+// C++ exceptions become Python ones; an argument the library refuses hands the call back (None).  Saving a
+// tensor runs the user's pack hooks, and what those raise has to come out as it is: torch.utils.checkpoint
+// ends its recomputation with an exception of its own.
 template <typename F>
 PyObject *guarded(F &&f) {
     try {
         return f();
     } catch (const Refused &) {
         Py_RETURN_NONE;
+    } catch (python_error &e) {
+        e.restore();
     } catch (const c10::OutOfMemoryError &e) {
         PyObject *torch = PyImport_ImportModule("torch");
         PyObject *type = torch ? PyObject_GetAttrString(torch, "OutOfMemoryError") : nullptr;

@@ -4,7 +4,7 @@ import torch
 import torch.autograd.forward_ad as fw
 
 from rgd_triton_b200 import ops
-from tests._util import gen, randn
+from tests._util import attention_backward, gen, randn, rotary_table
 
 pytestmark = pytest.mark.gpu
 
@@ -31,3 +31,58 @@ def test_forward_mode_is_refused_for_heads(op):
         dual = fw.make_dual(q, torch.ones_like(q))
         with pytest.raises(RuntimeError):
             ops.FusedHeadLayerNorm()(dual, k, False) if op == "headln" else ops.FlashAttention()(dual, k, v)
+
+
+# ---------------------------------------------------------------------------------------------- autograd around the calls
+def _calls():
+    """name -> (call, inputs that want a gradient): every operator on ordinary shapes of the native path."""
+    g = gen(3)
+    f16 = torch.float16
+    x, y = randn(g, 2, 9, 64).cuda(), randn(g, 2, 5, 96).cuda()
+    q, k = randn(g, 2, 40, 3, 64, dtype=f16).cuda(), randn(g, 2, 24, 3, 64, dtype=f16).cuda()
+    v = randn(g, 2, 24, 3, 64, dtype=f16).cuda()
+    bias = randn(g, 2, 3, 40, 24, dtype=f16).cuda()
+    pos = rotary_table(64, 32, f16).cuda()
+    rms, rms2 = ops.FusedRMSNorm(64).cuda(), ops.FusedRMSNorm2((64, 96)).cuda()
+    l2, l22, ln, rope, lnrope, attn = (ops.L2Normalize(), ops.FusedL2Normalize2(), ops.FusedHeadLayerNorm(), ops.RoPE(),
+                                       ops.FusedLNRoPE(), ops.FlashAttention())
+    return {"l2": (lambda a: l2(a), [x]), "l2x2": (lambda a, b: l22(a, b), [x, y]),
+            "rms": (lambda a: rms(a), [x]), "rms2": (lambda a, b: rms2(a, b), [x, y]),
+            "headln": (lambda a, b: ln(a, b, False), [q, k]), "rope": (lambda a, b: rope(a, b, pos, 20, False), [q, k]),
+            "lnrope": (lambda a, b: lnrope(a, b, pos, (20, 24), False), [q, k]),
+            "attn": (lambda a, b, c: attn(a, b, c), [q, k, v]), "attn_bias": (lambda a, b, c: attn(a, b, c, bias), [q, k, v])}
+
+
+CALLS = ["l2", "l2x2", "rms", "rms2", "headln", "rope", "lnrope", "attn", "attn_bias"]
+
+
+def _grads(call, inputs, wrap=lambda f: f):
+    leaves = [t.clone().requires_grad_(True) for t in inputs]
+    with attention_backward("two_kernel"):      # bit-reproducible, so that two ways can be compared exactly
+        out = wrap(call)(*leaves)
+        outs = out if isinstance(out, tuple) else (out,)
+        grads = torch.autograd.grad(outs, leaves, [torch.cos(o.detach().float()).to(o.dtype) for o in outs])
+    return [o.detach() for o in outs] + list(grads)
+
+
+@pytest.mark.parametrize("name", CALLS)
+def test_checkpoint(name):
+    """torch.utils.checkpoint stops its recomputation by an exception out of the pack hook of the region's last
+    saved tensor, which here is one of the operator's own."""
+    from torch.utils.checkpoint import checkpoint
+    call, inputs = _calls()[name]
+    want = _grads(call, inputs)
+    got = _grads(call, inputs, lambda f: lambda *a: checkpoint(f, *a, use_reentrant=False))
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("name", CALLS)
+def test_pack_hooks_raise_their_own_exception(name):
+    call, inputs = _calls()[name]
+
+    def pack(t):
+        raise KeyError("packed")
+    with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t):
+        with pytest.raises(KeyError, match="packed"):
+            call(*[t.clone().requires_grad_(True) for t in inputs])
