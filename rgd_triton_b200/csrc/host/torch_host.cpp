@@ -189,12 +189,23 @@ bool wants_grad(std::initializer_list<const Tensor *> ts) {
     return false;
 }
 
-// The gradient the engine hands over: undefined means zero; the kernels need a unit channel stride.
-Tensor upstream(const Tensor &g, const Tensor &ref) {
-    if (!g.defined()) return at::zeros(ref.sizes(), ref.options());
-    if (g.stride(-1) == 1) return g;
+// The kernels need a unit channel stride.
+Tensor unit(const Tensor &g) {
+    if (!g.defined() || g.stride(-1) == 1) return g;
     Tensor c = g.contiguous();
     return c.stride(-1) == 1 ? c : at::empty(g.sizes(), g.options()).copy_(g);
+}
+
+// The gradient the engine hands over: undefined means zero.
+Tensor upstream(const Tensor &g, const Tensor &ref) {
+    return g.defined() ? unit(g) : at::zeros(ref.sizes(), ref.options());
+}
+
+// What a backward unpacks may lie differently from what the forward saved: saved-tensor hooks move and copy
+// (torch.autograd.graph.save_on_cpu gives back a dense copy of a slice).  Strides are therefore taken from
+// the unpacked tensors, never kept from the forward; sizes and types have to be the same.
+void restored(bool ok, const char *what) {
+    TORCH_CHECK(ok, what, " backward: a saved tensor came back from its hooks with another shape, type or device");
 }
 
 template <typename N>
@@ -246,6 +257,7 @@ bool rows_ok(Rows &r) {
         if (i > 0 && (!plain(x, 3) || !like(x, a) || x.size(0) != r.B)) return false;
         r.N[i] = x.size(1);
         r.C[i] = x.size(2);
+        r.w_stride[i] = r.per_batch[i] = 0;
         const Tensor &w = r.w[i];
         if (!w.defined()) continue;
         if (!w.is_cuda() || w.device() != a.device() || code_of(w) < 0 || w.scalar_type() != r.w[0].scalar_type() ||
@@ -300,16 +312,25 @@ struct RowsBackward : public Node {
     }
     variable_list apply(variable_list &&grads) override {
         std::lock_guard<std::mutex> lock(mutex_);
-        Tensor xt[2], wt[2], dy[2], dx[2], dw[2];
+        Tensor dy[2], dx[2], dw[2];
         rgd_rows xs[2], dys[2], dxs[2];
         const void *ws[2] = {nullptr, nullptr};
         void *dws[2] = {nullptr, nullptr};
+        Rows r = this->r;       // with the unpacked tensors, and the weights' strides from them
+        Tensor(&xt)[2] = r.x, (&wt)[2] = r.w;
         for (int i = 0; i < r.n; ++i) {
             xt[i] = x[i].unpack();
             if (affine) wt[i] = w[i].unpack();
         }
         c10::cuda::OptionalCUDAGuard guard(xt[0].device());
         at::AutoDispatchBelowADInplaceOrView below;
+        for (int i = 0; i < r.n; ++i) {
+            xt[i] = unit(xt[i]);
+            wt[i] = unit(wt[i]);
+        }
+        restored(rows_ok(r) && r.dtype == this->r.dtype && std::equal(r.N, r.N + r.n, this->r.N) &&
+                     std::equal(r.C, r.C + r.n, this->r.C) && r.B == this->r.B && (!affine || r.w_dtype == this->r.w_dtype),
+                 affine ? "FusedRMSNorm" : "L2Normalize");
         for (int i = 0; i < r.n; ++i) {
             dy[i] = upstream(grads[i], xt[i]);
             dx[i] = new_like(xt[i]);
@@ -389,9 +410,9 @@ bool heads_ok(Heads &h, const Tensor &q, const Tensor &k) {
     return k.size(0) == h.B && k.size(head) == h.H && k.size(3) == h.d && h.d <= (h.op == HEAD_LN ? 256 : 128);
 }
 
-bool table_ok(Heads &h, const Tensor &q, const Tensor &pos) {
-    if (!plain(pos, 3) || pos.device() != q.device() || pos.size(0) != 2 || h.nq >= pos.size(1) || h.nk >= pos.size(1) ||
-        (pos.scalar_type() != q.scalar_type() && pos.scalar_type() != at::kFloat))
+bool table_ok(Heads &h, const Tensor &pos, c10::Device device) {
+    if (!plain(pos, 3) || pos.device() != device || pos.size(0) != 2 || h.nq >= pos.size(1) || h.nk >= pos.size(1) ||
+        (code_of(pos) != h.dtype && pos.scalar_type() != at::kFloat))
         return false;
     h.P = pos.size(1); h.R = pos.size(2); h.pos_s = pos.stride(0); h.pos_n = pos.stride(1);
     h.pos_dtype = code_of(pos);
@@ -468,6 +489,7 @@ struct HeadsBackward : public Node {
     variable_list apply(variable_list &&grads) override {
         std::lock_guard<std::mutex> lock(mutex_);
         Tensor qt, kt, pt;
+        Heads h = this->h;      // with the strides of the unpacked rotary table
         if (h.op != HEAD_ROPE) {
             qt = q.unpack();
             kt = k.unpack();
@@ -475,6 +497,15 @@ struct HeadsBackward : public Node {
         if (h.op != HEAD_LN) pt = pos.unpack();
         c10::cuda::OptionalCUDAGuard guard(options.device());
         at::AutoDispatchBelowADInplaceOrView below;
+        qt = unit(qt);
+        kt = unit(kt);
+        pt = unit(pt);
+        auto as_saved = [&](const Tensor &t, const std::vector<int64_t> &sizes) {
+            return plain(t, 4) && t.sizes() == at::IntArrayRef(sizes) && t.scalar_type() == options.dtype() && t.device() == options.device();
+        };
+        restored((h.op == HEAD_ROPE || (as_saved(qt, q_sizes) && as_saved(kt, k_sizes))) &&
+                     (h.op == HEAD_LN || (table_ok(h, pt, options.device()) && h.P == this->h.P && h.R == this->h.R &&
+                                          h.pos_dtype == this->h.pos_dtype)), name().c_str());
         Tensor g[2];
         for (int i = 0; i < 2; ++i) {
             if (!grads[i].defined()) g[i] = at::zeros(i ? k_sizes : q_sizes, options);
@@ -567,11 +598,22 @@ struct AttnBackward : public Node {
     }
     variable_list apply(variable_list &&grads) override {
         std::lock_guard<std::mutex> lock(mutex_);
-        const Tensor qt = q.unpack(), kt = k.unpack(), vt = v.unpack(), ot = o.unpack(shared_from_this()), lt = lse.unpack();
-        Tensor bt;
+        Tensor qt = q.unpack(), kt = k.unpack(), vt = v.unpack(), ot = o.unpack(shared_from_this()), lt = lse.unpack(), bt, tiles;
         if (a.bias_kind != RGD_BIAS_NONE) bt = bias.unpack();
         c10::cuda::OptionalCUDAGuard guard(qt.device());
         at::AutoDispatchBelowADInplaceOrView below;
+        for (Tensor *t : {&qt, &kt, &vt, &ot, &bt}) *t = unit(*t);
+        lt = lt.contiguous();
+        Attn a = this->a;       // with the strides of the unpacked bias
+        a.bias_kind = RGD_BIAS_NONE;
+        a.bias_dtype = RGD_F32;
+        restored(attn_ok(a, qt, kt, vt, bt) && a.B == this->a.B && a.H == this->a.H && a.tq == this->a.tq && a.tk == this->a.tk &&
+                     a.d == this->a.d && a.dtype == this->a.dtype && a.bias_kind == this->a.bias_kind &&
+                     a.bias_dtype == this->a.bias_dtype && plain(ot, 4) && like(ot, qt) && ot.sizes() == qt.sizes() &&
+                     lt.scalar_type() == at::kFloat && lt.device() == qt.device() && lt.dim() == 3 && lt.size(0) == a.B &&
+                     lt.size(1) == a.H && lt.size(2) == api.attn_lse_rows(a.tq), "FlashAttention");
+        // the tile lists are indexed by the bias's broadcast dimensions
+        if ((a.bias_sb == 0) == (this->a.bias_sb == 0) && (a.bias_sh == 0) == (this->a.bias_sh == 0)) tiles = this->tiles;
         const Tensor dot = upstream(grads[0], qt);
         Tensor dq = new_like(qt), dk = new_like(kt), dv = new_like(vt);
         int64_t bytes = std::max<int64_t>(api.attn_bwd_workspace_bytes(a.B, a.H, a.tq, a.tk, a.d, a.dtype), 16);
@@ -689,7 +731,7 @@ PyObject *py_rotary(PyObject *, PyObject *const *args, Py_ssize_t n) {
             if (PyErr_Occurred()) return nullptr;
         }
         h.heads_second = PyObject_IsTrue(args[2]);
-        if (!heads_ok(h, q, k) || !table_ok(h, q, pos) || !cutoffs(h, args[6]) || (at::GradMode::is_enabled() && pos.requires_grad()))
+        if (!heads_ok(h, q, k) || !table_ok(h, pos, q.device()) || !cutoffs(h, args[6]) || (at::GradMode::is_enabled() && pos.requires_grad()))
             Py_RETURN_NONE;
         return heads_call(h, q, k, pos);
     });

@@ -829,6 +829,11 @@ def _bias_tiles(cache, bias, bias_t, bias_s, q, seqlen_q, seqlen_k, causal):
     return None
 
 
+def _broadcast(bias, q):
+    """Over which of (batch, heads) the bias is broadcast: stride 0 there."""
+    return None if bias is None else tuple(s == 0 for s in bias.expand(q.shape[0], q.shape[2], -1, -1).stride()[:2])
+
+
 def _native_tiles(cache, bias, q, k, causal):
     """_bias_tiles for the native host path: the same policy, with the cheap refusals first so that an
     ordinary call does not describe its bias twice."""
@@ -877,7 +882,9 @@ class FlashAttnFunc(torch.autograd.Function):
         q, k, v, o, lse, bias_t, softmax_scale, tiles = _attn_forward(q, k, v, bias, causal, softmax_scale, kernel_cache)
         ctx.save_for_backward(q, k, v, o, lse, bias_t)
         ctx.causal, ctx.softmax_scale, ctx.kernel_cache = causal, softmax_scale, kernel_cache
-        ctx.tiles = tiles           # the backward of this call skips the same tiles
+        # the backward of this call skips the same tiles, if the bias is still broadcast over the dimensions by
+        # which their lists are indexed (saved-tensor hooks may have materialised it)
+        ctx.tiles, ctx.tiles_bcast = tiles, _broadcast(bias_t, q)
         ctx.mark_non_differentiable(lse)
         return o, lse
 
@@ -886,8 +893,8 @@ class FlashAttnFunc(torch.autograd.Function):
         q, k, v, o, lse, bias = ctx.saved_tensors
         cache = ctx.kernel_cache
         want_dbias = bias is not None and ctx.needs_input_grad[3]
-        dq, dk, dv, dbias = _attn_backward(q, k, v, bias, o, lse, do, ctx.causal, ctx.softmax_scale, cache, want_dbias,
-                                           ctx.tiles)
+        tiles = ctx.tiles if ctx.tiles_bcast == _broadcast(bias, q) else None
+        dq, dk, dv, dbias = _attn_backward(q, k, v, bias, o, lse, do, ctx.causal, ctx.softmax_scale, cache, want_dbias, tiles)
         if cache is not None:
             cache.bwd_odot = cache.bwd
         return dq, dk, dv, dbias, None, None, None
@@ -926,7 +933,7 @@ def _attn_backward(q, k, v, bias, o, lse, do, causal, softmax_scale, cache, want
     which the bias is broadcast; a vector bias's sum over the queries is formed inside the dK/dV
     kernel, a matrix bias's gradient is written by the dQ kernel."""
     do = _last_contig(do)
-    plan = _plan(cache, "bwd", _key(q, k, v, do, bias, extra=("attn", bool(causal), bool(want_dbias))),
+    plan = _plan(cache, "bwd", _key(q, k, v, o, do, bias, extra=("attn", bool(causal), bool(want_dbias))),
                  lambda: _require(do.shape == q.shape and do.dtype == q.dtype, "dO must match q"))
     lib = _lib.load()
     batch, seqlen_q, nheads, d = q.shape

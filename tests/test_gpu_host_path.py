@@ -3,7 +3,7 @@ import pytest
 import torch
 import torch.autograd.forward_ad as fw
 
-from rgd_triton_b200 import ops
+from rgd_triton_b200 import functional as F_, ops
 from tests._util import attention_backward, gen, randn, rotary_table
 
 pytestmark = pytest.mark.gpu
@@ -86,3 +86,70 @@ def test_pack_hooks_raise_their_own_exception(name):
     with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t):
         with pytest.raises(KeyError, match="packed"):
             call(*[t.clone().requires_grad_(True) for t in inputs])
+
+
+def _dense_copies(call, inputs):
+    """_grads with every saved tensor replaced by a dense copy of itself, as save_on_cpu does."""
+    with torch.autograd.graph.save_on_cpu():
+        return _grads(call, inputs)
+
+
+@pytest.mark.parametrize("name", ["rms", "rope", "lnrope", "attn_slice", "attn_transposed", "attn_q"])
+def test_saved_tensors_that_come_back_dense(name):
+    """Strided weights, rotary tables, biases and queries: the backward has to read the copies it unpacks by their
+    own strides."""
+    g = gen(6)
+    f16 = torch.float16
+    calls = _calls()
+    if name == "rms":
+        w = (1 + 0.1 * randn(g, 2, 3, 64)).cuda()[:, 1:2]           # [B, 1, C] of a [B, 3, C] modulation
+        m = ops.FusedRMSNorm(64, elementwise_affine=False)
+        call, inputs = lambda a, w: m(a, w), [calls["rms"][1][0], w]
+        base = _grads(call, [inputs[0], w.contiguous()])
+        got = _dense_copies(lambda a, big: m(a, big[:, 1:2]), [inputs[0], w.expand(2, 3, 64).contiguous()])
+        got[2] = got[2][:, 1:2]
+    elif name in ("rope", "lnrope"):
+        table = rotary_table(80, 48, f16).cuda()[:, 5:70, :32]
+        m = ops.RoPE() if name == "rope" else ops.FusedLNRoPE()
+        call, inputs = lambda a, b: m(a, b, table, 20, False), calls[name][1]
+        base, got = _grads(call, inputs), _dense_copies(call, inputs)
+    else:
+        m = ops.FlashAttention()
+        inputs = calls["attn"][1]
+        bias = {"attn_slice": randn(g, 2, 3, 64, 64, dtype=f16).cuda()[:, :, 8:48, 16:40],
+                "attn_transposed": randn(g, 3, 2, 40, 24, dtype=f16).cuda().transpose(0, 1), "attn_q": None}[name]
+        if name == "attn_q":
+            call = lambda a, b, c: m(a.transpose(1, 2).contiguous().transpose(1, 2), b, c)
+        else:
+            call = lambda a, b, c: m(a, b, c, bias)
+        base, got = _grads(call, inputs), _dense_copies(call, inputs)
+    for a, b in zip(got, base):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("native", [True, False])
+def test_tile_lists_of_a_bias_that_comes_back_dense(native, monkeypatch):
+    """An expanded bias has one slice of tile lists; its dense copy would index one per (batch, head)."""
+    if not native:
+        monkeypatch.setattr(F_, "_bind_host", lambda t: None)
+        monkeypatch.setattr(F_, "_HOST", None)
+    g = gen(7)
+    f16 = torch.float16
+    q, k, v = (randn(g, 2, 1024, 2, 64, dtype=f16).cuda() for _ in range(3))
+    bias = torch.zeros(1024, 1024, dtype=f16)
+    bias[:512, 512:] = -1e4
+    bias = bias.cuda().expand(2, 2, 1024, 1024)
+    m = ops.FlashAttention()
+    call = lambda a, b, c: m(a, b, c, bias)
+    base = [_grads(call, [q, k, v]) for _ in range(3)][-1]
+    assert torch.is_tensor(m.cache._tiles[2])
+    for a, b in zip(_dense_copies(call, [q, k, v]), base):
+        assert torch.equal(a, b)
+
+
+def test_saved_tensors_of_another_shape_are_refused():
+    call, inputs = _calls()["attn_bias"]
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t[..., :8] if t.dim() == 4 else t):
+        out = call(*[t.clone().requires_grad_(True) for t in inputs])
+        with pytest.raises(RuntimeError, match="saved tensor"):
+            out.sum().backward()
