@@ -11,6 +11,9 @@
 // caches that are not a _LaunchCache, a bias that wants a gradient.  The Python path in functional.py
 // handles those, so conditions here only have to be sufficient.
 //
+// Under compiled autograd a node is traced instead of run: its saved tensors are then stand-ins without
+// storage, and it calls the registered operator of its backward (rgd_triton_b200/library.py) on them.
+//
 // The C ABI is bound at run time through the handle of the library that _lib.py has loaded, so this
 // module has no link-time dependency on it and the two can never be different copies.
 #include <Python.h>
@@ -25,6 +28,7 @@
 #include <vector>
 
 #include <ATen/ATen.h>
+#include <ATen/core/dispatch/Dispatcher.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -34,6 +38,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/autograd/variable.h>
+#include <torch/csrc/dynamo/compiled_autograd.h>
 
 #include "../../../include/rgd_b200.h"
 
@@ -43,6 +48,8 @@ using at::Tensor;
 using torch::autograd::Node;
 using torch::autograd::SavedVariable;
 using torch::autograd::variable_list;
+using torch::dynamo::autograd::CompiledNodeArgs;
+using torch::dynamo::autograd::SwapSavedVariables;
 
 // ------------------------------------------------------------------ C ABI, bound once
 struct Api {
@@ -208,6 +215,45 @@ void restored(bool ok, const char *what) {
     TORCH_CHECK(ok, what, " backward: a saved tensor came back from its hooks with another shape, type or device");
 }
 
+// ------------------------------------------------------------------ compiled autograd
+bool stand_in(const Tensor &t) { return t.defined() && t.unsafeGetTensorImpl()->is_python_dispatch(); }
+
+// The operators are registered when their module is imported.
+void register_operators() {
+    PyGILState_STATE gil = PyGILState_Ensure();
+    PyObject *m = PyImport_ImportModule("rgd_triton_b200.library");
+    if (!m) PyErr_Clear();      // the lookup below then says what is missing
+    Py_XDECREF(m);
+    PyGILState_Release(gil);
+}
+
+template <typename... A>
+std::vector<c10::IValue> call_operator(const char *name, A &&...args) {
+    auto op = c10::Dispatcher::singleton().findSchemaOrThrow(name, "");
+    torch::jit::Stack stack{c10::IValue(std::forward<A>(args))...};
+    op.callBoxed(stack);
+    return stack;
+}
+
+// What compiled autograd asks of a node, given its attributes in a fixed order: SAVED lists the saved variables,
+// CONSTANTS what a traced backward is specialised on.
+#define RGD_COMPILED(SAVED, CONSTANTS)                                                                                \
+    void compiled_args(CompiledNodeArgs &args) const override {                                                       \
+        register_operators();                                                                                         \
+        auto collect = [&](const SavedVariable &v, bool is_output) { args.collect(v, is_output); };                  \
+        auto constant = [&](auto... v) { (args.collect(v), ...); };                                                  \
+        SAVED(collect)                                                                                                \
+        CONSTANTS(constant)                                                                                           \
+    }                                                                                                                 \
+    variable_list apply_with_saved(const variable_list &grads, SwapSavedVariables &saved) override {                 \
+        auto before = [&](SavedVariable &v, bool) { saved.before(v); };                                              \
+        auto after = [&](SavedVariable &v, bool) { saved.after(v); };                                                \
+        SAVED(before)                                                                                                 \
+        variable_list out = apply(variable_list(grads));                                                              \
+        SAVED(after)                                                                                                  \
+        return out;                                                                                                   \
+    }
+
 template <typename N>
 std::shared_ptr<N> new_node(torch::autograd::edge_list edges) {
     std::shared_ptr<N> n(new N(), torch::autograd::deleteNode);
@@ -310,6 +356,26 @@ struct RowsBackward : public Node {
             w[i].reset_data();
         }
     }
+#define RGD_SAVED(f)                      \
+    for (int i = 0; i < r.n; ++i) {       \
+        f(x[i], false);                   \
+        if (affine) f(w[i], false);       \
+    }
+#define RGD_CONSTANTS(f) f(r.n, affine, r.eps);
+    RGD_COMPILED(RGD_SAVED, RGD_CONSTANTS)
+#undef RGD_SAVED
+#undef RGD_CONSTANTS
+    variable_list traced(const variable_list &grads, const Tensor (&xt)[2], const Tensor (&wt)[2]) const {
+        c10::List<Tensor> xs, ws, dys;
+        for (int i = 0; i < r.n; ++i) {
+            xs.push_back(xt[i]);
+            if (affine) ws.push_back(wt[i]);
+            dys.push_back(grads[i].defined() ? grads[i].contiguous() : at::zeros_like(xt[i]));
+        }
+        const auto out = affine ? call_operator("rgd_b200::rmsnorm_bwd", xs, ws, dys, r.eps)
+                                : call_operator("rgd_b200::l2norm_bwd", xs, dys, r.eps);
+        return out.at(0).toTensorVector();
+    }
     variable_list apply(variable_list &&grads) override {
         std::lock_guard<std::mutex> lock(mutex_);
         Tensor dy[2], dx[2], dw[2];
@@ -322,6 +388,7 @@ struct RowsBackward : public Node {
             xt[i] = x[i].unpack();
             if (affine) wt[i] = w[i].unpack();
         }
+        if (stand_in(xt[0])) return traced(grads, xt, wt);
         c10::cuda::OptionalCUDAGuard guard(xt[0].device());
         at::AutoDispatchBelowADInplaceOrView below;
         for (int i = 0; i < r.n; ++i) {
@@ -486,6 +553,25 @@ struct HeadsBackward : public Node {
         k.reset_data();
         pos.reset_data();
     }
+#define RGD_SAVED(f)             \
+    if (h.op != HEAD_ROPE) {     \
+        f(q, false);             \
+        f(k, false);             \
+    }                            \
+    if (h.op != HEAD_LN) f(pos, false);
+#define RGD_CONSTANTS(f) f((int64_t)h.op, h.heads_second, h.cut_q, h.cut_k, h.eps, options, q_sizes, k_sizes);
+    RGD_COMPILED(RGD_SAVED, RGD_CONSTANTS)
+#undef RGD_SAVED
+#undef RGD_CONSTANTS
+    variable_list traced(const variable_list &grads, const Tensor &qt, const Tensor &kt, const Tensor &pt) const {
+        const Tensor dq = grads[0].defined() ? grads[0].contiguous() : at::zeros(q_sizes, options);
+        const Tensor dk = grads[1].defined() ? grads[1].contiguous() : at::zeros(k_sizes, options);
+        const auto out = h.op == HEAD_LN     ? call_operator("rgd_b200::headln_bwd", qt, kt, dq, dk, h.heads_second, h.eps)
+                         : h.op == HEAD_ROPE ? call_operator("rgd_b200::rope", dq, dk, pt, h.cut_q, h.cut_k, h.heads_second, true)
+                                             : call_operator("rgd_b200::lnrope_bwd", qt, kt, dq, dk, pt, h.cut_q, h.cut_k,
+                                                             h.heads_second, h.eps);
+        return {out.at(0).toTensor(), out.at(1).toTensor()};
+    }
     variable_list apply(variable_list &&grads) override {
         std::lock_guard<std::mutex> lock(mutex_);
         Tensor qt, kt, pt;
@@ -495,6 +581,7 @@ struct HeadsBackward : public Node {
             kt = k.unpack();
         }
         if (h.op != HEAD_LN) pt = pos.unpack();
+        if (stand_in(h.op == HEAD_LN ? qt : pt)) return traced(grads, qt, kt, pt);
         c10::cuda::OptionalCUDAGuard guard(options.device());
         at::AutoDispatchBelowADInplaceOrView below;
         qt = unit(qt);
@@ -596,10 +683,26 @@ struct AttnBackward : public Node {
         for (SavedVariable *s : {&q, &k, &v, &o, &lse, &bias}) s->reset_data();
         tiles.reset();
     }
+#define RGD_SAVED(f)             \
+    f(q, false);                 \
+    f(k, false);                 \
+    f(v, false);                 \
+    f(o, true);                  \
+    f(lse, false);               \
+    if (a.bias_kind != RGD_BIAS_NONE) f(bias, false);
+#define RGD_CONSTANTS(f) f(a.causal, a.scale, a.bias_kind);
+    RGD_COMPILED(RGD_SAVED, RGD_CONSTANTS)
+#undef RGD_SAVED
+#undef RGD_CONSTANTS
     variable_list apply(variable_list &&grads) override {
         std::lock_guard<std::mutex> lock(mutex_);
         Tensor qt = q.unpack(), kt = k.unpack(), vt = v.unpack(), ot = o.unpack(shared_from_this()), lt = lse.unpack(), bt, tiles;
         if (a.bias_kind != RGD_BIAS_NONE) bt = bias.unpack();
+        if (stand_in(qt)) {
+            const auto out = call_operator("rgd_b200::attn_bwd", qt, kt, vt, bt.defined() ? c10::IValue(bt) : c10::IValue(), ot, lt,
+                                           grads[0].defined() ? grads[0].contiguous() : at::zeros_like(qt), a.causal, a.scale, false);
+            return {out.at(0).toTensor(), out.at(1).toTensor(), out.at(2).toTensor()};
+        }
         c10::cuda::OptionalCUDAGuard guard(qt.device());
         at::AutoDispatchBelowADInplaceOrView below;
         for (Tensor *t : {&qt, &kt, &vt, &ot, &bt}) *t = unit(*t);

@@ -47,7 +47,7 @@ def _calls():
     l2, l22, ln, rope, lnrope, attn = (ops.L2Normalize(), ops.FusedL2Normalize2(), ops.FusedHeadLayerNorm(), ops.RoPE(),
                                        ops.FusedLNRoPE(), ops.FlashAttention())
     return {"l2": (lambda a: l2(a), [x]), "l2x2": (lambda a, b: l22(a, b), [x, y]),
-            "rms": (lambda a: rms(a), [x]), "rms2": (lambda a, b: rms2(a, b), [x, y]),
+            "rms": (rms, [x]), "rms2": (lambda a, b: rms2(a, b), [x, y]),
             "headln": (lambda a, b: ln(a, b, False), [q, k]), "rope": (lambda a, b: rope(a, b, pos, 20, False), [q, k]),
             "lnrope": (lambda a, b: lnrope(a, b, pos, (20, 24), False), [q, k]),
             "attn": (lambda a, b, c: attn(a, b, c), [q, k, v]), "attn_bias": (lambda a, b, c: attn(a, b, c, bias), [q, k, v])}
@@ -153,3 +153,31 @@ def test_saved_tensors_of_another_shape_are_refused():
         out = call(*[t.clone().requires_grad_(True) for t in inputs])
         with pytest.raises(RuntimeError, match="saved tensor"):
             out.sum().backward()
+
+
+# ---------------------------------------------------------------------------------------------- compiled autograd
+@pytest.mark.parametrize("name", CALLS)
+def test_compiled_autograd(name):
+    """Forward eagerly, backward traced by compiled autograd, also after a change of sizes and of a constant."""
+    from torch._dynamo import compiled_autograd
+
+    def grads(call, inputs, compiled):
+        leaves = [t.clone().requires_grad_(True) for t in inputs]
+        with attention_backward("two_kernel"):
+            out = call(*leaves)
+            outs = out if isinstance(out, tuple) else (out,)
+            gs = [torch.cos(o.detach().float()).to(o.dtype) for o in outs]
+            if compiled:
+                with compiled_autograd._enable(lambda gm: torch.compile(gm, backend="eager")):
+                    torch.autograd.backward(outs, gs)
+            else:
+                torch.autograd.backward(outs, gs)
+        return [t.grad for t in leaves]
+    call, inputs = _calls()[name]
+    smaller = inputs if name == "attn_bias" else [t[:, :5] for t in inputs]
+    pos = rotary_table(64, 32, torch.float16).cuda()
+    other = (lambda a, b: ops.RoPE()(a, b, pos, 3, False)) if name == "rope" else call
+    torch._dynamo.reset()
+    for f, ins in [(call, inputs), (call, smaller), (other, inputs)]:
+        for a, b in zip(grads(f, ins, True), grads(f, ins, False)):
+            assert torch.equal(a, b)
