@@ -8,7 +8,8 @@
 //
 // Every entry returns None for arguments it does not cover: anything that is wrong (the Python path then
 // raises the right exception), tensor subclasses, forward-mode tangents, views whose channel stride is not 1, empty tensors,
-// caches that are not a _LaunchCache, a bias that wants a gradient.  The Python path in functional.py
+// caches that are not a _LaunchCache, a bias that wants a gradient; and for every call while something watches
+// the operations (torch.jit.trace, dispatch modes, functorch transforms).  The Python path in functional.py
 // handles those, so conditions here only have to be sufficient.
 //
 // Under compiled autograd a node is traced instead of run: its saved tensors are then stand-ins without
@@ -28,8 +29,10 @@
 #include <vector>
 
 #include <ATen/ATen.h>
+#include <ATen/TracerMode.h>
 #include <ATen/core/dispatch/Dispatcher.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -213,6 +216,13 @@ Tensor upstream(const Tensor &g, const Tensor &ref) {
 // the unpacked tensors, never kept from the forward; sizes and types have to be the same.
 void restored(bool ok, const char *what) {
     TORCH_CHECK(ok, what, " backward: a saved tensor came back from its hooks with another shape, type or device");
+}
+
+// Something on this thread sees every operation (a tracer, a dispatch mode, a functorch transform) and would miss
+// this call: the Python functions take it.
+bool watched() {
+    return at::tracer::impl::is_dispatch_enabled() || c10::impl::TorchDispatchModeTLS::any_modes_set() ||
+           c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode);
 }
 
 // ------------------------------------------------------------------ compiled autograd
@@ -770,6 +780,7 @@ PyObject *attn_call(Attn &a, const Tensor &q, const Tensor &k, const Tensor &v, 
 template <typename F>
 PyObject *guarded(F &&f) {
     try {
+        if (watched()) Py_RETURN_NONE;
         return f();
     } catch (const Refused &) {
         Py_RETURN_NONE;

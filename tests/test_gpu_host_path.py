@@ -155,7 +155,7 @@ def test_saved_tensors_of_another_shape_are_refused():
             out.sum().backward()
 
 
-# ---------------------------------------------------------------------------------------------- compiled autograd
+# ---------------------------------------------------------------------------------------------- callers that watch the operations
 @pytest.mark.parametrize("name", CALLS)
 def test_compiled_autograd(name):
     """Forward eagerly, backward traced by compiled autograd, also after a change of sizes and of a constant."""
@@ -181,3 +181,36 @@ def test_compiled_autograd(name):
     for f, ins in [(call, inputs), (call, smaller), (other, inputs)]:
         for a, b in zip(grads(f, ins, True), grads(f, ins, False)):
             assert torch.equal(a, b)
+
+
+@pytest.mark.filterwarnings("ignore")       # of the tracer: sizes that become constants, its own deprecation
+@pytest.mark.parametrize("name", ["l2", "rms", "headln", "rope", "attn"])
+def test_jit_trace(name):
+    call, inputs = _calls()[name]
+    leaves = [t.clone().requires_grad_(True) for t in inputs]
+    traced = torch.jit.trace(call, tuple(leaves), check_trace=False)
+    fresh = [t.flip(1).clone() for t in inputs]
+    for a, b in zip(_grads(traced, fresh), _grads(call, fresh)):
+        assert torch.equal(a, b)
+
+
+def test_dispatch_modes_and_transforms():
+    """A dispatch mode sees the operator's allocations; a transform, which the operators have no rule for, is refused."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Seen(TorchDispatchMode):
+        def __init__(self):
+            super().__init__()
+            self.ops = []
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.ops.append(func)
+            return func(*args, **(kwargs or {}))
+    call, (x,) = _calls()["l2"]
+    with Seen() as seen:
+        y = call(x)
+    assert seen.ops and torch.equal(y, call(x))
+    with pytest.raises(RuntimeError):
+        torch.func.vmap(call)(x[None])
+    with pytest.raises(RuntimeError):
+        torch.func.grad(lambda t: call(t).sum())(x)
