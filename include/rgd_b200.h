@@ -276,7 +276,8 @@ int rgd_attn_fwd(const rgd_heads *q, const rgd_heads *k, const rgd_heads *v,
 /* Scratch bytes for rgd_attn_bwd: one fp32 row of delta = rowsum(O * dO) per
  * (batch, head) on the general path; on the tensor-memory path two fp32 rows
  * per (batch, head), lse * log2(e) and delta * scale, each Tq rounded up to
- * 128.  With exactly this much, no fp32 dQ accumulator is used on either path. */
+ * 128, which both paths reuse for the rows described at rgd_attn_bwd.  With exactly
+ * this much, no fp32 dQ accumulator is used on either path. */
 int64_t rgd_attn_bwd_workspace_bytes(int64_t B, int64_t H, int64_t Tq,
                                      int64_t Tk, int64_t d, int dtype);
 
@@ -299,7 +300,11 @@ int64_t rgd_attn_bwd_single_pass_workspace_bytes(int64_t B, int64_t H,
 /* dQ, dK, dV given dO.  Replaces _flash_attn_backward, including the
  * delta = rowsum(O * dO) pre-pass (flash_attn_triton_cached.py:885-1075).
  * The bias gradient (which the reference refuses, :1107) comes from
- * rgd_attn_bwd_dbias. */
+ * rgd_attn_bwd_dbias.
+ * A row whose every key carries a finite bias far below zero (log-sum-exp under
+ * -1e5) has the gradients of the probabilities its output was formed with: even
+ * over the keys with the largest bias once the scores are below that bias's
+ * rounding.  A row without any key (all -inf) passes no gradient on. */
 int rgd_attn_bwd(const rgd_heads *q, const rgd_heads *k, const rgd_heads *v,
                  const rgd_bias *bias, const rgd_heads *o, const float *lse,
                  const rgd_heads *d_o, const rgd_heads *dq,

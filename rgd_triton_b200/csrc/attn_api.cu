@@ -200,6 +200,12 @@ extern "C" int rgd_attn_bwd_dbias(const rgd_heads *q, const rgd_heads *k, const 
     fill_bwd(p, q, k, v, bias, o, d_o, dq, dk, dv, B, H, Tq, Tk, d, softmax_scale, causal);
     p.lse = const_cast<float *>(lse);
     p.delta = reinterpret_cast<float *>(workspace);
+    if (p.bias_kind != RGD_BIAS_NONE && (p.bias_f32 || dtype == RGD_BF16)) {    // no fp16 value masks a row so far
+        // general path: a far row's maximum over its delta, the sums in the second half of the workspace
+        p.far_m = p.delta;
+        p.far_l = p.delta + B * H * p.Tq_rounded;
+        p.far_ld = p.Tq_rounded;
+    }
     if (want_dbias && B > 0 && H > 0 && Tk > 0) {
         if (dbias->kind == RGD_BIAS_VECTOR &&
             cudaMemsetAsync(const_cast<void *>(dbias->ptr), 0, (size_t)(B * H * Tk) * sizeof(float), (cudaStream_t)stream) != cudaSuccess)

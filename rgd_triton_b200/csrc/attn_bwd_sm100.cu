@@ -32,6 +32,7 @@ namespace attn {
 using namespace rgd::sm100;
 
 int *tmem_status_ptr();   // attn_fwd_sm100.cu
+int far_rows_bwd(const AttnParams &p, int dtype, cudaStream_t st);      // attn_general.cu
 bool bias_tma_ok(const AttnParams &p);
 bool general_takes_bias(const AttnParams &p);
 int encode_bias_map(rgd_cache *cache, CUtensorMap *out, const AttnParams &p, bool bf16, int box_q);
@@ -2297,10 +2298,10 @@ __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __grid_constan
     if (l == 0 && i < Tq128) {
         const int64_t idx = (int64_t)bh * Tq128 + i;
         delta_s[idx] = a * p.scale;
-        // A row whose keys are all masked with a huge value (or -inf) has no P that lse still resolves
-        // (2^(x - lse2) would be inf or 0 by rounding): it passes no gradient on, like a row past the end.
+        // A row without any key passes no gradient on, like a row past the end; a far row neither, here: the
+        // general kernels add it afterwards (far_rows_bwd).
         const float lse = i < p.Tq ? p.lse[(int64_t)bh * p.Tq_rounded + i] : INFINITY;
-        lse2[idx] = lse < -1e7f ? INFINITY : lse * LOG2E;
+        lse2[idx] = lse == -INFINITY || (p.far_l != nullptr && far_row(lse)) ? INFINITY : lse * LOG2E;
     }
 }
 
@@ -2479,8 +2480,12 @@ int tmem_bwd(const AttnParams &p, int dtype, rgd_cache *cache, float *dq_acc, cu
     bp.d = p.d;
     bp.H = p.H; bp.Tq = p.Tq; bp.Tk = p.Tk; bp.Tq128 = Tq128; bp.causal = p.causal;
     bp.scale = p.scale; bp.scale_log2 = p.scale * LOG2E;
-    if (p.d > 64) return bf16 ? bwd_both<128, true>(bp, p, st) : bwd_both<128, false>(bp, p, st);
-    return bf16 ? bwd_both<64, true>(bp, p, st) : bwd_both<64, false>(bp, p, st);
+    const int rc = p.d > 64 ? (bf16 ? bwd_both<128, true>(bp, p, st) : bwd_both<128, false>(bp, p, st))
+                            : (bf16 ? bwd_both<64, true>(bp, p, st) : bwd_both<64, false>(bp, p, st));
+    if (rc != RGD_OK || p.far_l == nullptr) return rc;
+    AttnParams fp = p;      // the row statistics have been read: their place takes those of the far rows
+    fp.far_l = lse2; fp.far_m = delta_s; fp.far_ld = Tq128;
+    return far_rows_bwd(fp, dtype, st);
 }
 
 }  // namespace attn

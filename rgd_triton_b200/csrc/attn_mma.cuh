@@ -43,6 +43,12 @@ struct AttnParams {
     void *dbias;
     int64_t db_sb, db_sh, db_sq;
     int dbias_vec;                     // matrix form: rows are 16-byte addressable
+    // Far rows (backward only, see far_row): null when the bias cannot make any.  Per row, far_ld apart for each
+    // (batch, head): the largest score of a far row, and the sum of its exponentials relative to that (0 for a
+    // row that is not far; never 0 in the first row of a 64-row tile with a far row in it).  Written and read by
+    // attn_bwd_far (attn_general.cu) when the other kernels of the backward are done.
+    float *far_m, *far_l;
+    int far_ld;
     // Tile lists of a matrix bias (attn_tiles.cu), null when not given: which 128 x 128 tiles are
     // not entirely masked.  Used by the kernels that stage the bias by TMA, without a causal mask.
     const uint16_t *tiles;
@@ -77,6 +83,14 @@ inline TileLayout tile_layout(int64_t Bb, int64_t Hb, int64_t Tq, int64_t Tk) {
     L.total_bytes = L.words * 2 + (L.bitmap_bytes + 15) / 16 * 16;
     return L;
 }
+
+// A far row is one whose every key carries a large negative bias, so that its log-sum-exp, one fp32 number, no
+// longer resolves the probabilities: 2^(x - lse) is off by as much as half an ulp of lse * log2(e) (0.8 % at the
+// line below, a factor of 2^64 at a mask of -1e9).  Its probabilities are formed from the row's maximum and the sum
+// relative to it instead.  Rows above the line, those masked with -1e4 or an fp16 mask's lowest value among them,
+// and rows without any key (lse = -inf, all probabilities 0) are not far.
+constexpr float FAR_BELOW = -1e5f;
+__device__ __forceinline__ bool far_row(float lse) { return lse < FAR_BELOW && lse > -INFINITY; }
 
 template <typename T> struct Mma;
 template <> struct Mma<__half> {
@@ -150,10 +164,11 @@ __device__ __forceinline__ void load_tile(Tile<T, DPAD> &t, const T *g, int64_t 
 }
 
 // Store a warp's 16 x DPAD fp32 accumulator tile (C-fragment layout) to global
-// as T.  `g` points at (tile row 0, channel 0) of this warp's 16 rows.
+// as T.  `g` points at (tile row 0, channel 0) of this warp's 16 rows.  keep0 / keep8: whether this thread's two
+// rows are stored at all.
 template <typename T, int DPAD>
 __device__ __forceinline__ void store_acc(const float (&acc)[DPAD / 8][4], T *g, int64_t stride, int rows_valid, int d,
-                                          bool vec, float scale0, float scale8) {
+                                          bool vec, float scale0, float scale8, bool keep0 = true, bool keep8 = true) {
     const int lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
 #pragma unroll
     for (int nt = 0; nt < DPAD / 8; ++nt) {
@@ -163,7 +178,7 @@ __device__ __forceinline__ void store_acc(const float (&acc)[DPAD / 8][4], T *g,
             const int r = gq + half * 8;
             const float s = half ? scale8 : scale0;
             const float v0 = acc[nt][half * 2] * s, v1 = acc[nt][half * 2 + 1] * s;
-            if (r < rows_valid) {
+            if (r < rows_valid && (half ? keep8 : keep0)) {
                 T *p = g + (int64_t)r * stride + c;
                 if (vec && c + 1 < d) {   // 4-byte aligned: even channel, 8-element-aligned rows
                     *reinterpret_cast<uint32_t *>(p) = Mma<T>::pack(v0, v1);
@@ -174,6 +189,19 @@ __device__ __forceinline__ void store_acc(const float (&acc)[DPAD / 8][4], T *g,
             }
         }
     }
+}
+
+// The reverse: what is stored there is added to the accumulator tile.
+template <typename T, int DPAD>
+__device__ __forceinline__ void add_stored(float (&acc)[DPAD / 8][4], const T *g, int64_t stride, int rows_valid, int d) {
+    const int lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
+#pragma unroll
+    for (int nt = 0; nt < DPAD / 8; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int r = gq + (e >> 1) * 8, c = nt * 8 + 2 * tq + (e & 1);
+            if (r < rows_valid && c < d) acc[nt][e] += to_f32<T>(g[(int64_t)r * stride + c]);
+        }
 }
 
 // acc[8][4] (16 x 64) += A[16 x DPAD] * B[64 x DPAD]^T, both row-major in shared

@@ -99,20 +99,28 @@ inline TileOrder make_tile_order(int nblk, int BH, bool causal, int64_t bytes_pe
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <typename... Params, typename... Args>
-inline int launch_pdl(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
+inline int launch_pdl_cluster(void (*kernel)(Params...), dim3 grid, int cluster_x, int threads, size_t smem, cudaStream_t st,
+                              Args... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cudaLaunchAttribute attrs[2]{};
+    attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[0].val.programmaticStreamSerializationAllowed = 1;
+    attrs[1].id = cudaLaunchAttributeClusterDimension;
+    attrs[1].val.clusterDim.x = cluster_x;
+    attrs[1].val.clusterDim.y = attrs[1].val.clusterDim.z = 1;
+    cfg.attrs = attrs;
+    cfg.numAttrs = cluster_x > 1 ? 2 : 1;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
     count_launch();
     return cuda_status(e);
+}
+template <typename... Params, typename... Args>
+inline int launch_pdl(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
+    return launch_pdl_cluster(kernel, grid, 1, threads, smem, st, args...);
 }
 
 // ---------------------------------------------------------------------------

@@ -138,3 +138,62 @@ def test_largest_probability_is_not_rounded(tq, d):
     # What is left is the rounding of the output: within half an ulp, evenly spread, 2^-8 / sqrt(3) at the foot of a
     # binade and half of it at its top, 0.41 * 2^-8 in the mean square.  The lagging reference gave 0.97 * 2^-8.
     assert ((got - want) / want).pow(2).mean().sqrt() <= 0.55 * 2.0 ** -8
+
+
+def _masked_rows_reference(q, k, v, do, bias, causal, far):
+    """Output and gradients in 64 bits, with the probabilities of the rows in `far` even over their largest bias."""
+    q, k, v, do, bias = (t.double() for t in (q, k, v, do, bias))
+    scale = q.shape[-1] ** -0.5
+    bias = bias.expand(q.shape[0], q.shape[2], q.shape[1], k.shape[1])
+    if causal:
+        bias = bias.masked_fill(torch.ones(bias.shape[2:], dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    p = (torch.einsum("bqhd,bkhd->bhqk", q, k) * scale + bias).softmax(-1)
+    even = (bias == bias.amax(-1, keepdim=True)).double()
+    p = torch.where(far, even / even.sum(-1, keepdim=True), p)
+    o = torch.einsum("bhqk,bkhd->bqhd", p, v)
+    ds = p * (torch.einsum("bqhd,bkhd->bhqk", do, v) - torch.einsum("bqhd,bqhd->bhq", o, do)[..., None])
+    return (o, scale * torch.einsum("bhqk,bkhd->bqhd", ds, k), scale * torch.einsum("bhqk,bqhd->bkhd", ds, q),
+            torch.einsum("bhqk,bqhd->bkhd", p, do), ds)
+
+
+@pytest.mark.parametrize("mode", ["single_pass", "two_kernel"])
+@pytest.mark.parametrize("d", [20, 40, 64, 96, 128])
+@pytest.mark.parametrize("tq,tk,causal", [(5, 40, False), (130, 200, False), (200, 1, False), (70, 65, False), (130, 130, True)])
+@pytest.mark.parametrize("kind", ["vector", "matrix", "matrix_f32"])
+@pytest.mark.parametrize("mask", [-1e9, "lowest"])
+def test_gradients_of_rows_masked_far_down(mode, d, tq, tk, causal, kind, mask):
+    """Rows whose every key carries a mask so large that one fp32 log-sum-exp no longer resolves the probabilities:
+    all rows of a sequence, some rows of another (matrix bias), and rows in which one key carries it and the others
+    -inf.  Output and gradients are those of even probabilities over the largest bias, on every kernel."""
+    g = gen(d + tq)
+    B, H = 3, 2
+    q, k, v, do = (t.cuda() for t in _inputs(g, B, tq, tk, H, d, torch.bfloat16))
+    dt = torch.float32 if kind == "matrix_f32" else torch.bfloat16
+    low = torch.finfo(dt).min if mask == "lowest" else mask
+    bias = randn(g, B, 1, 1 if kind == "vector" else tq, tk, dtype=dt).cuda()
+    far = torch.zeros(B, 1, tq, 1, dtype=torch.bool, device="cuda")
+    bias[1], far[1] = low, True
+    if kind != "vector":
+        bias[0, :, 1:4], far[0, :, 1:4] = low, True
+    bias[2], far[2] = float("-inf"), True
+    bias[2, ..., 0 if causal else tk // 2] = low
+    want = _masked_rows_reference(q, k, v, do, bias, causal, far)
+    leaves = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    with attention_backward(mode):
+        o = F_.flash_attn_func(*leaves, bias, causal)
+        got = [o.detach(), *torch.autograd.grad(o, leaves, do)]
+    with_dbias = leaves + [bias.clone().requires_grad_(True)]
+    with attention_backward(mode):
+        o = F_.flash_attn_func(*with_dbias, causal)
+        grads = torch.autograd.grad(o, with_dbias, do)
+    for a, b in zip(got[1:], grads):
+        assert (a - b).float().norm() <= 1e-2 * b.float().norm() + 1e-4 * b.numel() ** 0.5
+    got.append(grads[3])
+    ds = want[4].sum(1, keepdim=True)
+    want = [*want[:4], ds.sum(2, keepdim=True) if kind == "vector" else ds]
+    for name, a, b in zip(("o", "dq", "dk", "dv", "dbias"), got, want):
+        for i in range(B):
+            # P and dS are rounded to bf16 (2^-9 in the mean square), the results once more; what cancels to nothing
+            # (dS of a row with one key) is left at the rounding of o in delta, 2^-9 of |dO| |o| per row
+            err, ref = (a[i].double() - b[i]).norm().item(), b[i].norm().item()
+            assert err <= 1e-2 * ref + 2e-3 * b[i].numel() ** 0.5 * (name != "o" and name != "dv"), (name, i, err, ref)
