@@ -282,8 +282,9 @@ int64_t rgd_attn_bwd_workspace_bytes(int64_t B, int64_t H, int64_t Tq,
                                      int64_t Tk, int64_t d, int dtype);
 
 /* Scratch bytes that select the single-pass backward (0 where there is none:
- * it exists for head_dim <= 64 on the tensor-memory path, without tile lists and
- * without a bias gradient): the bytes above, rounded up to 256, plus an fp32 dQ
+ * it exists on the tensor-memory path for head_dim 64, and for smaller multiples
+ * of 8 from 2^24 scores (B * H * Tq * Tk) on, without tile lists and without a bias
+ * gradient): the bytes above, rounded up to 256, plus an fp32 dQ
  * accumulator of B * H * Tq (rounded up to 128) * 64 elements, which the entry
  * point zeroes itself.  Given at least this much 256-byte aligned workspace,
  * rgd_attn_bwd evaluates S, dP and the exponentials once per tile pair and adds

@@ -15,7 +15,7 @@ int few_fwd(const AttnParams &p, int dtype, cudaStream_t st);
 bool tmem_bwd_eligible(const AttnParams &p);
 int tmem_bwd(const AttnParams &p, int dtype, rgd_cache *cache, float *dq_acc, cudaStream_t st);
 int64_t single_pass_acc_offset(int64_t B, int64_t H, int64_t Tq);
-int64_t single_pass_acc_bytes(int64_t B, int64_t H, int64_t Tq, int64_t d);
+int64_t single_pass_acc_bytes(int64_t B, int64_t H, int64_t Tq, int64_t Tk, int64_t d);
 int bounded_wait_selftest(int64_t limit_ns, cudaStream_t st);
 int64_t tmem_bwd_workspace_bytes(int64_t B, int64_t H, int64_t Tq);
 int build_bias_tiles(const void *bias, int64_t sb, int64_t sh, int64_t sq, int64_t Bb, int64_t Hb, int64_t Tq, int64_t Tk,
@@ -156,7 +156,7 @@ extern "C" int64_t rgd_attn_bwd_single_pass_workspace_bytes(int64_t B, int64_t H
                                                             int dtype) {
     const int64_t base = rgd_attn_bwd_workspace_bytes(B, H, Tq, Tk, d, dtype);
     if (base < 0) return base;
-    const int64_t acc = attn::single_pass_acc_bytes(B, H, Tq, d);
+    const int64_t acc = attn::single_pass_acc_bytes(B, H, Tq, Tk, d);
     if (acc == 0) return 0;
     return attn::single_pass_acc_offset(B, H, Tq) + acc;
 }

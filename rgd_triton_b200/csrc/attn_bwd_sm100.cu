@@ -2313,13 +2313,16 @@ int64_t tmem_bwd_workspace_bytes(int64_t B, int64_t H, int64_t Tq) {
     return 2 * B * H * Tq128 * (int64_t)sizeof(float);
 }
 
-// The fp32 dQ accumulator of the single-pass backward (0 bytes: no such form for this head_dim); it
-// follows the statistics rows in the workspace, 256-byte aligned.
+// The fp32 dQ accumulator of the single-pass backward (0 bytes: no such form for this shape); it
+// follows the statistics rows in the workspace, 256-byte aligned.  Smaller head dims have it only from
+// 2^24 scores on, where zero-padding them to 64 pays too: below that they would sum dQ in an order that
+// is not fixed where the general kernels do not, for a rounding to 64 channels that makes the accumulator
+// up to 8 times the data.
 int64_t single_pass_acc_offset(int64_t B, int64_t H, int64_t Tq) {
     return (tmem_bwd_workspace_bytes(B, H, Tq) + 255) / 256 * 256;
 }
-int64_t single_pass_acc_bytes(int64_t B, int64_t H, int64_t Tq, int64_t d) {
-    if (d < 8 || d > 64 || d % 8 != 0) return 0;
+int64_t single_pass_acc_bytes(int64_t B, int64_t H, int64_t Tq, int64_t Tk, int64_t d) {
+    if (d < 8 || d > 64 || d % 8 != 0 || (d != 64 && B * H * Tq * Tk < (int64_t)1 << 24)) return 0;
     const int64_t Tq128 = (Tq + 127) / 128 * 128;
     return B * H * Tq128 * 64 * (int64_t)sizeof(float);
 }

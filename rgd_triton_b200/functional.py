@@ -900,10 +900,10 @@ class FlashAttnFunc(torch.autograd.Function):
         return dq, dk, dv, dbias, None, None, None
 
 
-# How the attention backward forms dQ where the library offers a choice (head_dim up to 64 on
-# the tensor-memory kernels):
+# How the attention backward forms dQ where the library offers a choice (on the tensor-memory kernels:
+# head_dim 64, and smaller ones from 2^24 scores on):
 #   "single_pass"  S, dP and the exponentials are evaluated once per tile pair and the dQ partial tiles
-#                  are added into an fp32 accumulator (B * H * Tq * d * 4 bytes of scratch per call) with
+#                  are added into an fp32 accumulator (B * H * Tq * 64 * 4 bytes of scratch per call) with
 #                  vector reductions, like the reference's atomic adds into dq
 #                  (flash_attn_triton_cached.py:556-561): dK, dV bit-reproducible, dQ to its last bits only;
 #   "two_kernel"   a dK/dV kernel and a dQ kernel, every output bit-reproducible, no accumulator.

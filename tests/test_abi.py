@@ -111,3 +111,17 @@ def test_bias_gradient_and_tile_list_arguments_need_no_gpu(lib):
     big = _lib.Bias(None, 0, 0, 4096, _lib.RGD_BIAS_MATRIX, _lib.RGD_F16, None)
     assert L.rgd_attn_bias_tiles_build(ctypes.byref(big), 1, 1, 4096, 4096, -9984.0, buf, 64, None) == _lib.RGD_E_WORKSPACE
     assert L.rgd_attn_bias_tiles_build(ctypes.byref(mat), 1, 1, 4096, 4096, -9984.0, buf, 64, None) == _lib.RGD_E_STRIDE
+
+
+def test_single_pass_workspace_sizes():
+    """Where the single-pass backward exists: head_dim 64 at any size, smaller multiples of 8 from 2^24 scores on."""
+    from rgd_triton_b200 import _lib
+    lib = _lib.load()           # with the argument types declared
+    size = lambda B, H, Tq, Tk, d: lib.rgd_attn_bwd_single_pass_workspace_bytes(B, H, Tq, Tk, d, _lib.RGD_BF16)
+    base = lambda B, H, Tq, Tk, d: lib.rgd_attn_bwd_workspace_bytes(B, H, Tq, Tk, d, _lib.RGD_BF16)
+    assert size(1, 1, 100, 7, 64) == base(1, 1, 100, 7, 64) + 128 * 64 * 4
+    for d in (8, 40, 56):
+        assert size(1, 1, 4096, 4095, d) == 0
+        assert size(1, 1, 4096, 4096, d) == base(1, 1, 4096, 4096, d) + 4096 * 64 * 4
+    for d in (4, 60, 72, 128):
+        assert size(1, 1, 4096, 4096, d) == 0
