@@ -682,6 +682,17 @@ bool attn_ok(Attn &a, const Tensor &q, const Tensor &k, const Tensor &v, const T
     return true;
 }
 
+// Views that the aligned kernels take as they are, and the problems for which others are worth a dense copy
+// (functional.py, _addressable and flash_attn_func, which does the same for the inputs).
+bool addressable(const Tensor &t) {
+    bool ok = t.stride(-1) == 1 && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
+    for (int i = 0; i < 3; ++i) ok = ok && t.stride(i) % 8 == 0 && (t.stride(i) > 0 || t.size(i) == 1);
+    return ok;
+}
+bool copies_pay(const Attn &a) {
+    return a.d % 8 == 0 && a.d != 64 && a.d != 128 && a.B * a.H * a.tq * a.tk >= (int64_t)1 << 24;
+}
+
 struct AttnBackward : public Node {
     Attn a;
     SavedVariable q, k, v, o, lse, bias;
@@ -727,7 +738,8 @@ struct AttnBackward : public Node {
                      lt.size(1) == a.H && lt.size(2) == api.attn_lse_rows(a.tq), "FlashAttention");
         // the tile lists are indexed by the bias's broadcast dimensions
         if ((a.bias_sb == 0) == (this->a.bias_sb == 0) && (a.bias_sh == 0) == (this->a.bias_sh == 0)) tiles = this->tiles;
-        const Tensor dot = upstream(grads[0], qt);
+        Tensor dot = upstream(grads[0], qt);
+        if (copies_pay(a) && !addressable(dot)) dot = dot.clone(at::MemoryFormat::Contiguous);
         Tensor dq = new_like(qt), dk = new_like(kt), dv = new_like(vt);
         int64_t bytes = std::max<int64_t>(api.attn_bwd_workspace_bytes(a.B, a.H, a.tq, a.tk, a.d, a.dtype), 16);
         if (single_pass.load(std::memory_order_relaxed) && !tiles.defined())

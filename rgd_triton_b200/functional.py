@@ -933,6 +933,8 @@ def _attn_backward(q, k, v, bias, o, lse, do, causal, softmax_scale, cache, want
     which the bias is broadcast; a vector bias's sum over the queries is formed inside the dK/dV
     kernel, a matrix bias's gradient is written by the dQ kernel."""
     do = _last_contig(do)
+    if q.shape[-1] not in (64, 128) and q.shape[-1] % 8 == 0 and _pad_head_dim_pays(q, k) and not _addressable(do):
+        do = _dense(do)         # as for the inputs (flash_attn_func): o.sum(1) hands over a gradient of stride 0
     plan = _plan(cache, "bwd", _key(q, k, v, o, do, bias, extra=("attn", bool(causal), bool(want_dbias))),
                  lambda: _require(do.shape == q.shape and do.dtype == q.dtype, "dO must match q"))
     lib = _lib.load()
@@ -982,6 +984,17 @@ def _pad_head_dim_pays(q, k) -> bool:
         q.shape[0] * q.shape[2] * q.shape[1] * k.shape[1] >= (1 << 24)
 
 
+def _addressable(t, zero_strides=False) -> bool:
+    """Whether the aligned attention kernels take this view as it is: 16-byte rows, and positive strides (what is
+    expanded over batch or heads has stride 0; the few-query forward takes that too)."""
+    return t.stride(-1) == 1 and t.data_ptr() % 16 == 0 and all(
+        s % 8 == 0 and (s > 0 or n == 1 or zero_strides) for s, n in zip(t.stride()[:3], t.shape[:3]))
+
+
+def _dense(t):
+    return t.clone(memory_format=torch.contiguous_format)
+
+
 def flash_attn_func(q, k, v, bias=None, causal=False, softmax_scale=None, return_lse=False, kernel_cache=None):
     """q: (batch, seqlen_q, nheads, headdim); k, v: (batch, seqlen_k, nheads,
     headdim); bias: optional, 4-D, last two dims (1, seqlen_k) or (seqlen_q,
@@ -1008,6 +1021,12 @@ def flash_attn_func(q, k, v, bias=None, causal=False, softmax_scale=None, return
                               kernel_cache)
         o = res[0][..., :d].contiguous()
         return (o, res[1]) if return_lse else o
+    if d not in (0, 64, 128) and d % 8 == 0 and d < 128 and _pad_head_dim_pays(q, k):
+        # Large problems of these head dims are worth a dense copy of what is not addressable (keys shared by the
+        # heads, a slice at an odd offset): [2, 1100, 12, 96] with expanded keys and values 114 us on the general
+        # kernels without the copy.  Head dims 64 and 128 keep to the kernels that take the view as it is.
+        few = q.shape[1] <= 16 and not causal and not _needs_grad(q, k, v, bias)
+        q, k, v = (t if _addressable(t, few) else _dense(t) for t in (q, k, v))
     host = _HOST or _bind_host(q)
     if host is not None:
         tiles = _native_tiles(kernel_cache, bias, q, k, causal) if bias is not None else None

@@ -215,3 +215,32 @@ def test_small_problems_of_small_head_dims_are_reproducible(d, kind):
     for _ in range(5):
         for a, b in zip(run(), first):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("native", [True, False])
+@pytest.mark.parametrize("what", ["expanded", "odd_offset", "summed"])
+def test_large_problems_of_other_head_dims_copy_what_is_not_addressable(what, native, monkeypatch):
+    """Keys and values expanded over the heads, a slice at an odd offset, an upstream gradient of stride 0: the same
+    kernels run as on dense tensors, shown by the same bits."""
+    if not native:
+        monkeypatch.setattr(F_, "_bind_host", lambda t: None)
+        monkeypatch.setattr(F_, "_HOST", None)
+    g = gen(96)
+    B, T, H, d = 2, 840, 12, 96
+    q, k, v = (randn(g, B, T, H, d, dtype=torch.bfloat16).cuda() for _ in range(3))
+    do = randn(g, B, T, H, d, dtype=torch.bfloat16).cuda()
+    if what == "expanded":
+        k, v = (t[:, :, :1].expand(B, T, H, d) for t in (k, v))
+    elif what == "odd_offset":
+        q = torch.cat([q.flatten(), q.flatten()[:8]])[1:-7].view(B, T, H, d)
+    else:
+        do = do[:, :1].expand(B, T, H, d)
+
+    def run(dense):
+        leaves = [(t.clone(memory_format=torch.contiguous_format) if dense else t.detach()).requires_grad_(True)
+                  for t in (q, k, v)]
+        with attention_backward("two_kernel"):
+            o = F_.flash_attn_func(*leaves)
+            return [o.detach(), *torch.autograd.grad(o, leaves, do.contiguous() if dense else do)]
+    for a, b in zip(run(False), run(True)):
+        assert torch.equal(a, b)
