@@ -146,7 +146,10 @@ __global__ void __launch_bounds__(FEW_WARPS * 32) attn_few_kernel(const __grid_c
                 const int key = key0 + t * 8 + tq * 2 + (e & 1), r = gq + (e >> 1) * 8;
                 float x = s[t][e] * fp.scale_log2;
                 if constexpr (BIAS)
-                    if (key < p.Tk && r < p.Tq) x += bias_log2(bias_at_t<T>(p, bias_bh, r, key));
+                    if (key < p.Tk && r < p.Tq) {
+                        const float bv = bias_at_t<T>(p, bias_bh, r, key);
+                        x += p.bias_f32 ? bias_log2<float>(bv) : bias_log2<T>(bv);
+                    }
                 if (key >= p.Tk) x = -INFINITY;
                 s[t][e] = x;
                 mx[e >> 1] = fmaxf(mx[e >> 1], x);

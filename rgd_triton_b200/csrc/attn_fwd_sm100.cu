@@ -101,7 +101,7 @@ __device__ __forceinline__ void bias_from_smem(const unsigned char *tile, int ro
         union { uint4 u; T v[8]; } cv;
         cv.u = *reinterpret_cast<const uint4 *>(rowp + (((c0 + i) ^ (row_l & 7)) << 4));
 #pragma unroll
-        for (int e = 0; e < 8; ++e) b[8 * i + e] = BF16 ? bias_log2(to_f32<T>(cv.v[e])) : to_f32<T>(cv.v[e]) * LOG2E;
+        for (int e = 0; e < 8; ++e) b[8 * i + e] = bias_log2<T>(to_f32<T>(cv.v[e]));
     }
 }
 
@@ -134,11 +134,12 @@ __device__ __forceinline__ void load_bias32(const FwdTmaParams &p, const char *b
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const float4 v = reinterpret_cast<const float4 *>(src)[i];
-                b[4 * i] = bias_log2(v.x); b[4 * i + 1] = bias_log2(v.y); b[4 * i + 2] = bias_log2(v.z); b[4 * i + 3] = bias_log2(v.w);
+                b[4 * i] = bias_log2<float>(v.x); b[4 * i + 1] = bias_log2<float>(v.y);
+                b[4 * i + 2] = bias_log2<float>(v.z); b[4 * i + 3] = bias_log2<float>(v.w);
             }
         } else {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) b[i] = (col0 + i < p.Tk) ? bias_log2(src[i]) : 0.f;
+            for (int i = 0; i < 32; ++i) b[i] = (col0 + i < p.Tk) ? bias_log2<float>(src[i]) : 0.f;
         }
     } else {
         const T *src = reinterpret_cast<const T *>(bias_bh) + off;
@@ -147,11 +148,11 @@ __device__ __forceinline__ void load_bias32(const FwdTmaParams &p, const char *b
             for (int i = 0; i < 4; ++i) {
                 const Vec<T, 8> v = load_vec<T, 8>(src + 8 * i);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) b[8 * i + e] = bias_log2(to_f32<T>(v.v[e]));
+                for (int e = 0; e < 8; ++e) b[8 * i + e] = bias_log2<T>(to_f32<T>(v.v[e]));
             }
         } else {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) b[i] = (col0 + i < p.Tk) ? bias_log2(to_f32<T>(src[i])) : 0.f;
+            for (int i = 0; i < 32; ++i) b[i] = (col0 + i < p.Tk) ? bias_log2<T>(to_f32<T>(src[i])) : 0.f;
         }
     }
 }
@@ -520,7 +521,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) attn_fwd_tmem(const __grid_con
                     if (kj < p.Tk)
                         bvl = p.bias_f32 ? reinterpret_cast<const float *>(bias_bh)[kj]
                                          : to_f32<T>(reinterpret_cast<const T *>(bias_bh)[kj]);
-                    sm.vbias[t][j & 1][row_l] = bias_log2(bvl);
+                    sm.vbias[t][j & 1][row_l] = p.bias_f32 ? bias_log2<float>(bvl) : bias_log2<T>(bvl);
                     mbar_arrive(&sm.vb_ready[t]);
                 }
             }

@@ -4,6 +4,8 @@
 // take (head_dim not a multiple of 8, unaligned strides).
 #pragma once
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace rgd {
@@ -15,9 +17,16 @@ constexpr int NTHREADS = 128;   // 4 warps, 16 tile rows each
 constexpr int PAD = 8;          // 16-byte row padding: conflict-free ldmatrix
 constexpr float LOG2E = 1.4426950408889634f;
 
-// bias * log2(e), rounded towards zero: a mask near the lowest fp32 / bf16 value stays finite, so that a row
-// whose keys are all masked with it is uniform and not empty; -inf stays -inf.
-__device__ __forceinline__ float bias_log2(float b) { return __fmul_rz(b, LOG2E); }
+// bias * log2(e).  From bf16 or fp32 (T the type the value was stored in) rounded towards zero, so that a mask near the
+// type's lowest value stays finite and a row whose keys are all masked with it is even and not empty (-inf stays
+// -inf), with the next constant above LOG2E: 6.9e-8 above log2(e), it centres the truncation, and the product is within
+// 6.9e-8 of the exact one, where LOG2E rounded to nearest is within 7.3e-8.  No fp16 value overflows.
+template <typename T>
+__device__ __forceinline__ float bias_log2(float b) {
+    constexpr float ABOVE = 1.44269514083862304f;       // LOG2E + 2^-23
+    if constexpr (std::is_same<T, __half>::value) return b * LOG2E;
+    else return __fmul_rz(b, ABOVE);
+}
 // Internal answer of the tensor-memory entry points: nothing was launched, run the general kernels.
 constexpr int TMEM_NOT_TAKEN = -1000;
 

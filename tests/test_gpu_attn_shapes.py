@@ -244,3 +244,22 @@ def test_large_problems_of_other_head_dims_copy_what_is_not_addressable(what, na
             return [o.detach(), *torch.autograd.grad(o, leaves, do.contiguous() if dense else do)]
     for a, b in zip(run(False), run(True)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("tq", [5, 130])
+@pytest.mark.parametrize("kind", ["vector", "matrix", "matrix_odd"])
+@pytest.mark.parametrize("dt,bias_dt", [("f16", "f16"), ("bf16", "bf16"), ("f16", "f32"), ("bf16", "f32")])
+def test_bias_conversion_is_as_exact_as_one_rounding(tq, kind, dt, bias_dt):
+    """One visible key and no score: the log-sum-exp is the key's bias, taken to base 2 and back."""
+    g = gen(tq)
+    B, H, tk = 8, 50, 9 if kind == "matrix_odd" else 8
+    q, k, v, _ = (t.cuda() for t in _inputs(g, B, tq, tk, H, 64, DTYPES[dt]))
+    value = (randn(g, B, H, 1 if kind == "vector" else tq) * 100).to(DTYPES[bias_dt])
+    value[value == 0] = 1
+    bias = torch.full((*value.shape, tk), float("-inf"), dtype=value.dtype)
+    bias[..., 3] = value
+    _, lse = F_.flash_attn_func(torch.zeros_like(q), k, v, bias.cuda(), return_lse=True)
+    value = value.double().expand(B, H, tq)
+    # the product is within 7.3e-8 (constant and rounding) of the exact one, the constant of the way back 0.3e-8 off,
+    # its product rounded to 6.0e-8
+    assert ((lse[:, :, :tq].cpu().double() - value) / value).abs().max() <= 1.37e-7
