@@ -554,9 +554,8 @@ struct HeadsBackward : public Node {
     std::vector<int64_t> q_sizes, k_sizes;      // for upstream gradients that are undefined (zero)
     at::TensorOptions options;
 
-    std::string name() const override {
-        return h.op == HEAD_LN ? "FusedHeadLayerNormBackward" : h.op == HEAD_ROPE ? "RoPEBackward" : "FusedLNRoPEBackward";
-    }
+    const char *operator_name() const { return h.op == HEAD_LN ? "FusedHeadLayerNorm" : h.op == HEAD_ROPE ? "RoPE" : "FusedLNRoPE"; }
+    std::string name() const override { return std::string(operator_name()) + "Backward"; }
     void release_variables() override {
         std::lock_guard<std::mutex> lock(mutex_);
         q.reset_data();
@@ -602,7 +601,7 @@ struct HeadsBackward : public Node {
         };
         restored((h.op == HEAD_ROPE || (as_saved(qt, q_sizes) && as_saved(kt, k_sizes))) &&
                      (h.op == HEAD_LN || (table_ok(h, pt, options.device()) && h.P == this->h.P && h.R == this->h.R &&
-                                          h.pos_dtype == this->h.pos_dtype)), name().c_str());
+                                          h.pos_dtype == this->h.pos_dtype)), operator_name());
         Tensor g[2];
         for (int i = 0; i < 2; ++i) {
             if (!grads[i].defined()) g[i] = at::zeros(i ? k_sizes : q_sizes, options);
@@ -683,10 +682,10 @@ bool attn_ok(Attn &a, const Tensor &q, const Tensor &k, const Tensor &v, const T
 }
 
 // Views that the aligned kernels take as they are, and the problems for which others are worth a dense copy
-// (functional.py, _addressable and flash_attn_func, which does the same for the inputs).
-bool addressable(const Tensor &t) {
+// (functional.py, _addressable and flash_attn_func, which makes those of the inputs).
+bool addressable(const Tensor &t, bool zero_strides = false) {
     bool ok = t.stride(-1) == 1 && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
-    for (int i = 0; i < 3; ++i) ok = ok && t.stride(i) % 8 == 0 && (t.stride(i) > 0 || t.size(i) == 1);
+    for (int i = 0; i < 3; ++i) ok = ok && t.stride(i) % 8 == 0 && (t.stride(i) > 0 || t.size(i) == 1 || zero_strides);
     return ok;
 }
 bool copies_pay(const Attn &a) {
@@ -873,6 +872,10 @@ PyObject *py_attn(PyObject *, PyObject *const *args, Py_ssize_t n) {
             Py_RETURN_NONE;
         if (!attn_ok(a, q, k, v, bias) || (bias.defined() && at::GradMode::is_enabled() && bias.requires_grad())) Py_RETURN_NONE;
         a.causal = PyObject_IsTrue(args[6]);
+        if (copies_pay(a)) {
+            const bool few = a.tq <= 16 && !a.causal && !wants_grad({&q, &k, &v});
+            if (!addressable(q, few) || !addressable(k, few) || !addressable(v, few)) Py_RETURN_NONE;
+        }
         a.scale = args[7] == Py_None ? 0.0 : PyFloat_AsDouble(args[7]);
         if (PyErr_Occurred()) return nullptr;
         if (a.scale == 0.0) a.scale = 1.0 / sqrt((double)a.d);

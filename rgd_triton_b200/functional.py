@@ -1021,18 +1021,26 @@ def flash_attn_func(q, k, v, bias=None, causal=False, softmax_scale=None, return
                               kernel_cache)
         o = res[0][..., :d].contiguous()
         return (o, res[1]) if return_lse else o
-    if d not in (0, 64, 128) and d % 8 == 0 and d < 128 and _pad_head_dim_pays(q, k):
-        # Large problems of these head dims are worth a dense copy of what is not addressable (keys shared by the
-        # heads, a slice at an odd offset): [2, 1100, 12, 96] with expanded keys and values 114 us on the general
-        # kernels without the copy.  Head dims 64 and 128 keep to the kernels that take the view as it is.
-        few = q.shape[1] <= 16 and not causal and not _needs_grad(q, k, v, bias)
-        q, k, v = (t if _addressable(t, few) else _dense(t) for t in (q, k, v))
     host = _HOST or _bind_host(q)
     if host is not None:
-        tiles = _native_tiles(kernel_cache, bias, q, k, causal) if bias is not None else None
+        tiles, seen = None, None
+        if bias is not None:
+            seen = getattr(kernel_cache, "_tiles", None)
+            tiles = _native_tiles(kernel_cache, bias, q, k, causal)
         out = host.attn(kernel_cache, q, k, v, bias, tiles, causal, softmax_scale, return_lse)
         if out is not None:
             return out
+        if bias is not None and kernel_cache is not None:
+            kernel_cache._tiles = seen          # what follows counts this call's sight of the bias itself
+    if d not in (0, 64, 128) and d % 8 == 0 and d < 128 and _pad_head_dim_pays(q, k):
+        # Large problems of these head dims are worth a dense copy of what is not addressable (keys shared by the
+        # heads, a slice at an odd offset; the native path hands them back): [2, 1100, 12, 96] with expanded keys
+        # and values 114 us on the general kernels without the copy, 46 with it.  Head dims 64 and 128 keep to the
+        # kernels that take the view as it is.
+        few = q.shape[1] <= 16 and not causal and not _needs_grad(q, k, v, bias)
+        dense = [t if _addressable(t, few) else _dense(t) for t in (q, k, v)]
+        if any(a is not b for a, b in zip(dense, (q, k, v))):
+            return flash_attn_func(*dense, bias, causal, softmax_scale, return_lse, kernel_cache)
     if not _needs_grad(q, k, v, bias):
         _, _, _, o, lse, _, _, _ = _attn_forward(q, k, v, bias, causal, softmax_scale, kernel_cache)
     else:

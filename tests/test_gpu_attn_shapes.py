@@ -263,3 +263,16 @@ def test_bias_conversion_is_as_exact_as_one_rounding(tq, kind, dt, bias_dt):
     # the product is within 7.3e-8 (constant and rounding) of the exact one, the constant of the way back 0.3e-8 off,
     # its product rounded to 6.0e-8
     assert ((lse[:, :, :tq].cpu().double() - value) / value).abs().max() <= 1.37e-7
+
+
+def test_a_bias_is_not_scanned_on_its_first_call():
+    """Also where the call passes through the dispatch twice (keys and values that are copied first)."""
+    from rgd_triton_b200 import ops
+    g = gen(1)
+    q = randn(g, 2, 1024, 8, 96, dtype=torch.float16).cuda()
+    k, v = (randn(g, 2, 1024, 1, 96, dtype=torch.float16).cuda().expand(2, 1024, 8, 96) for _ in range(2))
+    bias = torch.full((1, 1, 1024, 1024), -1e4, dtype=torch.float16).triu(1).cuda()
+    m = ops.FlashAttention()
+    for sight in range(3):
+        m(q, k, v, bias)
+        assert torch.is_tensor(m.cache._tiles[2]) == (sight > 0)
