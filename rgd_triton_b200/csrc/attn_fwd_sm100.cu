@@ -519,9 +519,9 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) attn_fwd_tmem(const __grid_con
                     const int kj = j * TN + row_l;
                     float bvl = 0.f;
                     if (kj < p.Tk)
-                        bvl = p.bias_f32 ? reinterpret_cast<const float *>(bias_bh)[kj]
-                                         : to_f32<T>(reinterpret_cast<const T *>(bias_bh)[kj]);
-                    sm.vbias[t][j & 1][row_l] = p.bias_f32 ? bias_log2<float>(bvl) : bias_log2<T>(bvl);
+                        bvl = p.bias_f32 ? bias_log2<float>(reinterpret_cast<const float *>(bias_bh)[kj])
+                                         : bias_log2<T>(to_f32<T>(reinterpret_cast<const T *>(bias_bh)[kj]));
+                    sm.vbias[t][j & 1][row_l] = bvl;
                     mbar_arrive(&sm.vb_ready[t]);
                 }
             }
