@@ -61,6 +61,13 @@ class _LaunchCache:
     def __getstate__(self):
         return {k: v for k, v in vars(self).items() if not k.startswith("_plan_") and k not in ("_tiles", "_state")}
 
+    def __setstate__(self, state):
+        # A cache that was saved before the slots lived in the native state holds them as attributes, next to
+        # "_native": their names are kept, what they held says nothing about this process.
+        if "_fields" not in state:
+            state = {"_fields": tuple(k for k in state if not k.startswith("_"))}
+        self.__dict__.update(state)
+
     def __deepcopy__(self, memo):
         new = _LaunchCache(())
         new.__dict__.update(self.__getstate__())

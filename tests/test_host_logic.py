@@ -135,3 +135,19 @@ def test_package_exports():
     for n in ("FlashAttention", "L2Normalize", "FusedL2Normalize2", "FusedHeadLayerNorm", "FusedRMSNorm",
               "FusedRMSNorm2", "RoPE", "FusedLNRoPE", "CachableModule"):
         assert hasattr(R, n)
+
+
+def test_launch_cache_saved_by_an_earlier_version_loads():
+    """Such a cache held its slots as attributes (empty, or a launch key) beside "_native"."""
+    import copy
+    import pickle
+
+    from rgd_triton_b200.ops import _LaunchCache
+    old = _LaunchCache.__new__(_LaunchCache)
+    old.__setstate__({"fwd": (((2, 9, 64), (576, 64, 1)), "l2"), "bwd": None, "_native": None})
+    for cache in (old, copy.deepcopy(old), pickle.loads(pickle.dumps(old))):
+        assert cache.fwd is None and cache.bwd is None
+        assert repr(cache) == "LaunchCache(fwd=None, bwd=None)"
+        assert cache.stats() == (0, 0, 0)
+    with pytest.raises(AttributeError):
+        old.nothing
