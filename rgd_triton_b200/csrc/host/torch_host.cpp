@@ -186,6 +186,13 @@ bool state_of(PyObject *cache, State &out) {
     return ok;
 }
 
+// bool(o); what its __bool__ raises goes to the caller.
+bool truth(PyObject *o) {
+    const int v = PyObject_IsTrue(o);
+    if (v < 0) throw python_error();
+    return v == 1;
+}
+
 bool tensor_arg(PyObject *o, Tensor &out) {
     if (!THPVariable_CheckExact(o)) return false;
     out = THPVariable_Unpack(o);
@@ -837,7 +844,7 @@ PyObject *py_headln(PyObject *, PyObject *const *args, Py_ssize_t n) {
         if (n != 5 || !state_of(args[0], h.state) || !tensor_arg(args[3], q) || !tensor_arg(args[4], k)) Py_RETURN_NONE;
         h.eps = PyFloat_AsDouble(args[1]);
         if (PyErr_Occurred()) return nullptr;
-        h.heads_second = PyObject_IsTrue(args[2]);
+        h.heads_second = truth(args[2]);
         if (!heads_ok(h, q, k)) Py_RETURN_NONE;
         return heads_call(h, q, k, Tensor());
     });
@@ -855,7 +862,7 @@ PyObject *py_rotary(PyObject *, PyObject *const *args, Py_ssize_t n) {
             h.eps = PyFloat_AsDouble(args[1]);
             if (PyErr_Occurred()) return nullptr;
         }
-        h.heads_second = PyObject_IsTrue(args[2]);
+        h.heads_second = truth(args[2]);
         if (!heads_ok(h, q, k) || !table_ok(h, pos, q.device()) || !cutoffs(h, args[6]) || (at::GradMode::is_enabled() && pos.requires_grad()))
             Py_RETURN_NONE;
         return heads_call(h, q, k, pos);
@@ -871,7 +878,7 @@ PyObject *py_attn(PyObject *, PyObject *const *args, Py_ssize_t n) {
             (args[4] != Py_None && !tensor_arg(args[4], bias)) || (args[5] != Py_None && !tensor_arg(args[5], tiles)))
             Py_RETURN_NONE;
         if (!attn_ok(a, q, k, v, bias) || (bias.defined() && at::GradMode::is_enabled() && bias.requires_grad())) Py_RETURN_NONE;
-        a.causal = PyObject_IsTrue(args[6]);
+        a.causal = truth(args[6]);
         if (copies_pay(a)) {
             const bool few = a.tq <= 16 && !a.causal && !wants_grad({&q, &k, &v});
             if (!addressable(q, few) || !addressable(k, few) || !addressable(v, few)) Py_RETURN_NONE;
@@ -879,7 +886,7 @@ PyObject *py_attn(PyObject *, PyObject *const *args, Py_ssize_t n) {
         a.scale = args[7] == Py_None ? 0.0 : PyFloat_AsDouble(args[7]);
         if (PyErr_Occurred()) return nullptr;
         if (a.scale == 0.0) a.scale = 1.0 / sqrt((double)a.d);
-        return attn_call(a, q, k, v, bias, tiles, PyObject_IsTrue(args[8]));
+        return attn_call(a, q, k, v, bias, tiles, truth(args[8]));
     });
 }
 

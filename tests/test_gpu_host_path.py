@@ -214,3 +214,14 @@ def test_dispatch_modes_and_transforms():
         torch.func.vmap(call)(x[None])
     with pytest.raises(RuntimeError):
         torch.func.grad(lambda t: call(t).sum())(x)
+
+
+@pytest.mark.parametrize("arg", ["causal", "heads_second"])
+def test_flags_without_a_truth_value(arg):
+    """What bool() of the argument raises is what the call raises."""
+    q, k, v = _calls()["attn"][1]
+    with pytest.raises(RuntimeError, match="[Bb]oolean value"):
+        if arg == "causal":
+            ops.FlashAttention()(q, k, v, None, torch.tensor([True, False]))
+        else:
+            ops.FusedHeadLayerNorm()(q, q, torch.tensor([True, False]))
