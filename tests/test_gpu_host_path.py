@@ -225,3 +225,107 @@ def test_flags_without_a_truth_value(arg):
             ops.FlashAttention()(q, k, v, None, torch.tensor([True, False]))
         else:
             ops.FusedHeadLayerNorm()(q, q, torch.tensor([True, False]))
+
+
+# ---------------------------------------------------------------------------------------------- the native path against the Python one
+ROUTES = ["native", "no_cache", "python"]
+
+
+def _by_route(route, monkeypatch):
+    """The same operators through the native path, without launch caches, or through the Python functions."""
+    calls = _calls()
+    if route == "no_cache":
+        for call, _ in calls.values():
+            for m in [call] + [c.cell_contents for c in (getattr(call, "__closure__", None) or ())]:
+                if isinstance(m, ops.CachableModule):
+                    m.enable_cache(False)
+    if route == "python":
+        monkeypatch.setattr(F_, "_bind_host", lambda t: None)
+        monkeypatch.setattr(F_, "_HOST", None)
+    return calls
+
+
+@pytest.mark.parametrize("route", ROUTES[1:])
+@pytest.mark.parametrize("name", CALLS)
+def test_routes_agree(name, route, monkeypatch):
+    """Checks, marshalling and workspaces exist twice, in C++ and in Python: same bits, dense and strided."""
+    call, inputs = _calls()[name]
+    strided = [torch.cat([t, t], dim=-2)[..., : t.shape[-2], :] for t in inputs]
+    want = [_grads(call, ins) for ins in (inputs, strided)]
+    other = _by_route(route, monkeypatch)[name][0]
+    for ins, w in zip((inputs, strided), want):
+        for a, b in zip(_grads(other, ins), w):
+            assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("route", ROUTES)
+@pytest.mark.parametrize("name", CALLS)
+def test_two_backwards(name, route, monkeypatch):
+    """A kept graph gives the same gradients again; a released one, and inputs changed in between, are errors."""
+    call, inputs = _by_route(route, monkeypatch)[name]
+    leaves = [t.clone().requires_grad_(True) for t in inputs]
+    with attention_backward("two_kernel"):
+        out = call(*leaves)
+        outs = out if isinstance(out, tuple) else (out,)
+        gs = [torch.ones_like(o) for o in outs]
+        first = torch.autograd.grad(outs, leaves, gs, retain_graph=True)
+        second = torch.autograd.grad(outs, leaves, gs)
+    for a, b in zip(first, second):
+        assert torch.equal(a, b)
+    with pytest.raises(RuntimeError, match="second time"):
+        torch.autograd.grad(outs, leaves, gs)
+    if name != "rope":              # saves no input
+        out = call(*leaves)
+        outs = out if isinstance(out, tuple) else (out,)
+        with torch.no_grad():
+            leaves[0].mul_(2)
+        with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+            torch.autograd.grad(outs, leaves, gs)
+
+
+@pytest.mark.parametrize("route", ROUTES)
+@pytest.mark.parametrize("name", ["l2x2", "rms2", "headln", "rope", "lnrope"])
+def test_one_of_two_outputs_without_a_gradient(name, route, monkeypatch):
+    """The input whose output nobody used gets zeros, the other one its gradient."""
+    call, inputs = _by_route(route, monkeypatch)[name]
+    leaves = [t.clone().requires_grad_(True) for t in inputs]
+    outs = call(*leaves)
+    g = torch.cos(outs[1].detach().float()).to(outs[1].dtype)
+    used = torch.autograd.grad(outs[1], leaves, g)
+    outs = call(*leaves)
+    both = torch.autograd.grad(outs, leaves, [torch.zeros_like(outs[0]), g])
+    assert not used[0].any()
+    for a, b in zip(used, both):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("route", ROUTES)
+def test_side_stream_and_thread(route, monkeypatch):
+    """Forward and backward on a stream of their own, from another thread, through one module used by both threads."""
+    import threading
+    calls = _by_route(route, monkeypatch)
+    want = {n: _grads(*calls[n]) for n in ("rms", "lnrope", "attn_bias")}
+    torch.cuda.synchronize()
+    failures = []
+
+    def work():
+        try:
+            stream = torch.cuda.Stream()
+            for _ in range(5):
+                for n, w in want.items():
+                    with torch.cuda.stream(stream):
+                        leaves = [t.clone().requires_grad_(True) for t in calls[n][1]]
+                        out = calls[n][0](*leaves)
+                        outs = out if isinstance(out, tuple) else (out,)
+                        got = [*outs, *torch.autograd.grad(outs, leaves, [torch.cos(o.detach().float()).to(o.dtype) for o in outs])]
+                    stream.synchronize()
+                    assert all(torch.equal(a, b) for a, b in zip(got, w))
+        except BaseException as e:      # noqa: BLE001  (reported by the main thread)
+            failures.append(e)
+    with attention_backward("two_kernel"):
+        threads = [threading.Thread(target=work) for _ in range(2)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    assert not failures
