@@ -42,6 +42,7 @@ from __future__ import annotations
 import ctypes as C
 import math
 import os
+import threading
 import weakref
 
 import torch
@@ -84,19 +85,21 @@ def _plan(cache, slot: str, key, validate):
     returned and host-side validation is skipped; otherwise `validate()` runs,
     the slot takes the new key and a fresh, empty plan.  The plan is a dict in
     which the launch helpers keep their marshalled ctypes arguments, so a
-    repeated call only refreshes the data pointers.  Without a cache every call
+    repeated call only refreshes the data pointers.  A plan belongs to the thread
+    that made it: another one, which could refresh the same pointers between this
+    thread's refresh and its launch, makes its own.  Without a cache every call
     validates and marshals from scratch (returns None)."""
     if cache is None:
         validate()
         return None
-    store = cache.__dict__
+    store, thread = cache.__dict__, threading.get_ident()
     ent = store.get("_plan_" + slot)
-    if ent is not None and ent[0] == key:
+    if ent is not None and ent[0] == key and ent[2] == thread:
         return ent[1]
     validate()
     setattr(cache, slot, key)
     plan = {}
-    store["_plan_" + slot] = (key, plan)
+    store["_plan_" + slot] = (key, plan, thread)
     return plan
 
 

@@ -151,3 +151,17 @@ def test_launch_cache_saved_by_an_earlier_version_loads():
         assert cache.stats() == (0, 0, 0)
     with pytest.raises(AttributeError):
         old.nothing
+
+
+def test_launch_plans_belong_to_one_thread():
+    """The marshalled arguments of a plan are refreshed before every launch: two threads must not share them."""
+    import threading
+
+    cache = ops._LaunchCache(("fwd",))
+    mine = F_._plan(cache, "fwd", ("key",), lambda: None)
+    assert F_._plan(cache, "fwd", ("key",), lambda: None) is mine
+    theirs = []
+    t = threading.Thread(target=lambda: theirs.append(F_._plan(cache, "fwd", ("key",), lambda: None)))
+    t.start()
+    t.join()
+    assert theirs[0] is not mine and F_._plan(cache, "fwd", ("key",), lambda: None) is not theirs[0]
