@@ -276,3 +276,57 @@ def test_a_bias_is_not_scanned_on_its_first_call():
     for sight in range(3):
         m(q, k, v, bias)
         assert torch.is_tensor(m.cache._tiles[2]) == (sight > 0)
+
+
+@pytest.mark.parametrize("d,H", [(128, 100), (64, 200)])
+def test_causal_grid_of_more_heads_than_a_group_of_long_queries(d, H):
+    """As above for the dK/dV kernel, whose groups are sized by Q and dO: 95 / 190 heads of 1030 queries fit one."""
+    g = gen(H + 1)
+    q, k, v, do = (t.cuda() for t in _inputs(g, 1, 1030, 300, H, d, torch.bfloat16))
+
+    def run(sl):
+        a, b, c = (t[:, :, sl].contiguous().requires_grad_(True) for t in (q, k, v))
+        o = F_.flash_attn_func(a, b, c, None, True)
+        return (o.detach(), *torch.autograd.grad(o, (a, b, c), do[:, :, sl].contiguous()))
+    with attention_backward("two_kernel"):
+        whole = run(slice(0, H))
+        halves = [run(slice(0, H // 2)), run(slice(H // 2, H))]
+    for w, x, y in zip(whole, *halves):
+        assert torch.equal(w, torch.cat([x, y], dim=2))
+
+
+@pytest.mark.parametrize("d,single", [(d, False) for d in (8, 24, 56, 72, 104, 120)] + [(d, True) for d in (8, 24, 56)])
+@pytest.mark.parametrize("kind", [None, "vector", "matrix"])
+def test_nothing_is_written_past_the_channels(d, single, kind):
+    """Outputs whose rows lie 8 elements further apart than they are long: the gaps and both ends stay as they
+    were, forward (few and many queries) and backward."""
+    import ctypes as C
+    lib, bf = _lib.load(), torch.bfloat16
+    g = gen(d)
+    # with 2^24 scores and more the single-pass form exists for these head dims
+    for B, H, tq, tk in ([(1, 2, 2900, 2896)] if single else [(2, 3, 5, 40), (2, 3, 130, 136)]):
+        q, k, v, do = (t.cuda() for t in _inputs(g, B, tq, tk, H, d, bf))
+        bias = None if kind is None else make_bias(g, kind, B, H, tq, tk, bf).cuda()
+        bias_s = F_._prep_bias(bias, q, tq, tk)[1]
+        lse = torch.empty(B, H, lib.rgd_attn_lse_rows(tq), device="cuda")
+        bufs = [torch.full((B * n * H * (d + 8) + 16,), 7.0, dtype=bf, device="cuda") for n in (tq, tq, tk, tk)]
+        outs = [b[8:-8].view(B, n, H, d + 8)[..., :d] for b, n in zip(bufs, (tq, tq, tk, tk))]
+        ref = lambda t: C.byref(F_._attn_heads(t))
+        o, dq, dk, dv = outs
+        stream = torch.cuda.current_stream().cuda_stream
+        assert lib.rgd_attn_fwd(ref(q), ref(k), ref(v), C.byref(bias_s), ref(o), lse.data_ptr(), B, H, tq, tk, d, d ** -0.5, 0,
+                                _lib.RGD_BF16, None, stream) == 0
+        size = lib.rgd_attn_bwd_single_pass_workspace_bytes if single else lib.rgd_attn_bwd_workspace_bytes
+        work = torch.empty(size(B, H, tq, tk, d, _lib.RGD_BF16), dtype=torch.uint8, device="cuda")
+        assert lib.rgd_attn_bwd(ref(q), ref(k), ref(v), C.byref(bias_s), ref(o), lse.data_ptr(), ref(do), ref(dq), ref(dk),
+                                ref(dv), B, H, tq, tk, d, d ** -0.5, 0, _lib.RGD_BF16, work.data_ptr(), work.numel(), None,
+                                stream) == 0
+        leaves = [t.clone().requires_grad_(True) for t in (q, k, v)]
+        with attention_backward("single_pass" if single else "two_kernel"):
+            want = F_.flash_attn_func(*leaves, bias)
+            grads = torch.autograd.grad(want, leaves, do)
+        for i, (a, b) in enumerate(zip(outs, (want, *grads))):
+            # dQ of the single-pass form is summed in no fixed order: one rounding step of the largest value
+            assert torch.equal(a, b) or (single and i == 1 and (a - b).abs().max() <= 2.0 ** -8 * b.abs().max())
+        for b, n in zip(bufs, (tq, tq, tk, tk)):
+            assert (b[:8] == 7).all() and (b[-8:] == 7).all() and (b[8:-8].view(B, n, H, d + 8)[..., d:] == 7).all()
