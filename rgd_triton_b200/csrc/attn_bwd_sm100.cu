@@ -68,23 +68,16 @@ struct BwdTmaParams {
     // slice the query blocks to visit (dK/dV kernel), per query block the key blocks (dQ kernel)
     const uint16_t *tlk_cnt, *tlk_list, *tlq_cnt, *tlq_list;
     int tl_nqb, tl_nkb;
-    float *dq_acc;                      // single-pass form (head_dim 64): fp32 dQ accumulator [B, H, 16, Tq128, 4], else null
+    float *dq_acc;                      // single-pass form (head_dim up to 64): fp32 dQ accumulator [B, H, 16, Tq128, 4], else null
 };
 
-// BSTAGES: stages of TMA-staged bias tiles (query rows x key columns, 16-bit, two
-// 64-column panels with 128-byte swizzle); 0 when the bias does not go through TMA.
-template <int D, int BSTAGES>
+template <int D>
 struct alignas(1024) BwdTmaSmem {
     unsigned char x1[BT * D * 2], x2[BT * D * 2];            // fixed tiles
     unsigned char y1[2][BT * D * 2], y2[2][BT * D * 2];      // looped tiles, 2 stages
-    unsigned char bias[BSTAGES > 0 ? BSTAGES : 1][BSTAGES > 0 ? BT * BT * 2 : 1024];
-    // dK/dV: row statistics of the staged query block (not with head_dim 128 and staged bias
-    // tiles: shared memory is full there and the statistics are read from global memory)
-    static constexpr int NSTAT = (D == 128 && BSTAGES > 0) ? 4 : BT;
-    alignas(16) float lse_s[2][NSTAT], dsc_s[2][NSTAT];
+    alignas(16) float lse_s[2][BT], dsc_s[2][BT];            // dK/dV: row statistics of the staged query block
     uint64_t x_full, g1_full, g2_full, p_ready, ds_ready, acc_full;
     uint64_t y_full[2], y_empty[2];
-    uint64_t bb_full[2], bb_empty[2];
     uint32_t tmem_base;
 };
 
@@ -104,15 +97,10 @@ __device__ __forceinline__ uint32_t pack16b(float a, float b) {
     }
 }
 
-// BIAS: whether an additive bias exists; the no-bias instantiation carries none of
-// the bias code (and none of its register pressure).
-// (BIAS: 0 none, 1 read from global memory by the compute threads, 2 staged through TMA.)
-
-template <int D, bool BF16, bool DKDV, int BIAS>
+// A matrix bias that TMA cannot stage (fp32, or rows that are not 16-byte addressable): the compute threads read it
+// from global memory.  DKDV: the dK/dV kernel, else dQ.
+template <int D, bool BF16, bool DKDV>
 __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_tmem(const __grid_constant__ BwdTmaParams p) {
-    constexpr int BSTAGES = BIAS == 2 ? (D == 64 ? 2 : 1) : 0;
-    constexpr bool STAGE_STATS = DKDV && !(D == 128 && BSTAGES > 0);
-    constexpr uint32_t BIAS_BYTES = BT * BT * 2;
     constexpr int HALVES = D / 64;
     constexpr uint32_t PANEL = 128 * 64 * 2;
     constexpr uint32_t TILE_BYTES = BT * D * 2;
@@ -121,7 +109,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_tmem(const __grid_con
     using T = typename std::conditional<BF16, __nv_bfloat16, __half>::type;
 
     extern __shared__ unsigned char smem_raw[];
-    BwdTmaSmem<D, BSTAGES> &sm = *reinterpret_cast<BwdTmaSmem<D, BSTAGES> *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    BwdTmaSmem<D> &sm = *reinterpret_cast<BwdTmaSmem<D> *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int blk, bh;
@@ -151,8 +139,6 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_tmem(const __grid_con
         for (int s = 0; s < 2; ++s) {
             mbar_init(&sm.y_full[s], 1);
             mbar_init(&sm.y_empty[s], 1);
-            mbar_init(&sm.bb_full[s], 1);
-            mbar_init(&sm.bb_empty[s], 256);
         }
         fence_mbar_init();
     }
@@ -166,7 +152,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_tmem(const __grid_con
     const uint32_t tbase = sm.tmem_base;
     if (DKDV) {
         grid_wait();        // the row statistics are in place
-        grid_trigger();     // the dQ kernel needs nothing from this one: it may fill the SMs this grid leaves idle
+        grid_trigger();     // after the wait: see attn_bwd_dkdv_sub
     }
 
     if (warp == 8) {
@@ -178,7 +164,6 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_tmem(const __grid_con
             tma_prefetch_desc(mx2);
             tma_prefetch_desc(my1);
             tma_prefetch_desc(my2);
-            if constexpr (BIAS == 2) tma_prefetch_desc(&p.mbias);
             mbar_expect_tx(&sm.x_full, 2 * TILE_BYTES);
             for (int hh = 0; hh < HALVES; ++hh) {
                 tma_load_4d(sm.x1 + hh * PANEL, mx1, &sm.x_full, hh * 64, r0, h, b);
@@ -190,27 +175,16 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_tmem(const __grid_con
                 const uint32_t ph = (uint32_t)(it >> 1) & 1u;
                 ok = mbar_wait(&sm.y_empty[s], ph ^ 1u, status, 41);
                 if (!ok) break;
-                mbar_expect_tx(&sm.y_full[s], 2 * TILE_BYTES + (STAGE_STATS ? 2 * BT * 4 : 0));
+                mbar_expect_tx(&sm.y_full[s], 2 * TILE_BYTES + (DKDV ? 2 * BT * 4 : 0));
                 const int row = (i_begin + it) * BT;
                 for (int hh = 0; hh < HALVES; ++hh) {
                     tma_load_4d(sm.y1[s] + hh * PANEL, my1, &sm.y_full[s], hh * 64, row, h, b);
                     tma_load_4d(sm.y2[s] + hh * PANEL, my2, &sm.y_full[s], hh * 64, row, h, b);
                 }
-                if constexpr (STAGE_STATS) {
+                if constexpr (DKDV) {
                     // the query block's lse / delta rows, read by every compute thread in both phases
                     bulk_load_1d(sm.lse_s[s], p.lse2 + (int64_t)bh * p.Tq128 + row, BT * 4, &sm.y_full[s]);
                     bulk_load_1d(sm.dsc_s[s], p.delta_s + (int64_t)bh * p.Tq128 + row, BT * 4, &sm.y_full[s]);
-                }
-                if constexpr (BIAS == 2) {
-                    const int sb = it % BSTAGES;
-                    ok = mbar_wait(&sm.bb_empty[sb], ((uint32_t)(it / BSTAGES) & 1u) ^ 1u, status, 42);
-                    if (!ok) break;
-                    mbar_expect_tx(&sm.bb_full[sb], BIAS_BYTES);
-                    // tile rows are queries, columns keys
-                    const int qrow = DKDV ? row : r0, kcol = DKDV ? r0 : row;
-                    for (int pn = 0; pn < 2; ++pn)
-                        tma_load_4d(sm.bias[sb] + pn * (BT * 128), &p.mbias, &sm.bb_full[sb], kcol + pn * 64, qrow,
-                                    p.bias_h0 ? 0 : h, p.bias_b0 ? 0 : b);
                 }
             }
             if (!ok)
@@ -279,10 +253,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_tmem(const __grid_con
         const uint32_t lane_base = tbase + ((uint32_t)((warp & 3) * 32) << 16);
         const float *lse2_bh = p.lse2 + (int64_t)bh * p.Tq128;
         const float *ds_bh = p.delta_s + (int64_t)bh * p.Tq128;
-        const char *bias_bh = nullptr;
-        if constexpr (BIAS == 1)
-            bias_bh = reinterpret_cast<const char *>(p.bias) +
-                      ((int64_t)b * p.b_sb + (int64_t)h * p.b_sh) * (p.bias_f32 ? 4 : 2);
+        const char *bias_bh = reinterpret_cast<const char *>(p.bias) +
+                              ((int64_t)b * p.b_sb + (int64_t)h * p.b_sh) * (p.bias_f32 ? 4 : 2);
 
         // DQ: per-thread row statistics (rows past Tq hold +inf / 0, so they yield P = 0)
         float lse_row = INFINITY, dsc_row = 0.f;
@@ -301,78 +273,44 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_tmem(const __grid_con
             // mask, and any block touching the end of the keys.  Rows / columns past
             // the end of the QUERIES need nothing: their lse2 is +inf.
             const bool diag = p.causal && (DKDV ? (blk0 == r0) : (blk0 + BT > r0));
-            const bool slow = BIAS != 0 || diag || cta_key_tail || (!DKDV && blk0 + BT > p.Tk);
             float pv[64];
 
             // Bias for this thread's 64 elements, fetched before waiting for the score tile so
             // the loads overlap the wait.  Indices are clamped to stay in bounds; elements
             // past the ends are masked below.
-            float bv[BIAS != 0 ? 64 : 1];
-            if constexpr (BIAS == 2) {
-                const int sb = it % BSTAGES;
-                ok = mbar_wait(&sm.bb_full[sb], (uint32_t)(it / BSTAGES) & 1u, status, 65);
-                if (!ok) break;
-                const unsigned char *tile = sm.bias[sb];
-                if (DKDV) {
-                    // thread = key column row_l of the tile, 64 query rows half*64 .. +63
-                    const unsigned char *colp = tile + (row_l >> 6) * (BT * 128) + (row_l & 7) * 2;
-                    const int kc = (row_l & 63) >> 3;
+            float bv[64];
+            if (DKDV) {
+                const int kj = min(row, p.Tk - 1);
 #pragma unroll
-                    for (int i = 0; i < 64; ++i) {
-                        const int qr = half * 64 + i;
-                        bv[i] = to_f32<T>(*reinterpret_cast<const T *>(colp + qr * 128 + ((kc ^ (qr & 7)) << 4)));
-                    }
-                } else {
-                    // thread = query row row_l, 64 key columns = the whole 128-byte row of panel `half`
-                    const unsigned char *rowp = tile + half * (BT * 128) + row_l * 128;
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        union { uint4 u; T v[8]; } cv;
-                        cv.u = *reinterpret_cast<const uint4 *>(rowp + ((c ^ (row_l & 7)) << 4));
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) bv[8 * c + e] = to_f32<T>(cv.v[e]);
-                    }
+                for (int i = 0; i < 64; ++i) {
+                    const int qi = min(c0 + i, p.Tq - 1);
+                    const int64_t off = (int64_t)qi * p.b_sq + kj;
+                    bv[i] = p.bias_f32 ? __ldg(reinterpret_cast<const float *>(bias_bh) + off)
+                                       : to_f32<T>(reinterpret_cast<const T *>(bias_bh)[off]);
                 }
-                // (the stage is handed back at the end of the iteration, once instructions that
-                // consume these values have been issued: an arrive right here could be performed
-                // while the loads above are still in flight, and with a single stage the refill
-                // by the copy engine follows at once)
-            }
-            if constexpr (BIAS == 1) {
-                if (DKDV) {
-                    const int kj = min(row, p.Tk - 1);
+            } else {
+                const int qi = min(row, p.Tq - 1);
+                const int64_t off = (int64_t)qi * p.b_sq + c0;
+                if (!p.bias_f32 && p.bias_vec && c0 + 64 <= p.Tk) {
+                    const T *src = reinterpret_cast<const T *>(bias_bh) + off;
 #pragma unroll
-                    for (int i = 0; i < 64; ++i) {
-                        const int qi = min(c0 + i, p.Tq - 1);
-                        const int64_t off = (p.bias_kind == RGD_BIAS_MATRIX ? (int64_t)qi * p.b_sq : 0) + kj;
-                        bv[i] = p.bias_f32 ? __ldg(reinterpret_cast<const float *>(bias_bh) + off)
-                                           : to_f32<T>(reinterpret_cast<const T *>(bias_bh)[off]);
+                    for (int i = 0; i < 8; ++i) {
+                        const Vec<T, 8> v = load_vec<T, 8>(src + 8 * i);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) bv[8 * i + e] = to_f32<T>(v.v[e]);
                     }
                 } else {
-                    const int qi = min(row, p.Tq - 1);
-                    const int64_t off = (p.bias_kind == RGD_BIAS_MATRIX ? (int64_t)qi * p.b_sq : 0) + c0;
-                    if (!p.bias_f32 && p.bias_vec && c0 + 64 <= p.Tk) {
-                        const T *src = reinterpret_cast<const T *>(bias_bh) + off;
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            const Vec<T, 8> v = load_vec<T, 8>(src + 8 * i);
-#pragma unroll
-                            for (int e = 0; e < 8; ++e) bv[8 * i + e] = to_f32<T>(v.v[e]);
-                        }
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 64; ++i) {
-                            const int64_t o2 = off + min(i, p.Tk - 1 - c0 < 0 ? 0 : p.Tk - 1 - c0);
-                            bv[i] = p.bias_f32 ? __ldg(reinterpret_cast<const float *>(bias_bh) + o2)
-                                               : to_f32<T>(reinterpret_cast<const T *>(bias_bh)[o2]);
-                        }
+                    for (int i = 0; i < 64; ++i) {
+                        const int64_t o2 = off + min(i, p.Tk - 1 - c0 < 0 ? 0 : p.Tk - 1 - c0);
+                        bv[i] = p.bias_f32 ? __ldg(reinterpret_cast<const float *>(bias_bh) + o2)
+                                           : to_f32<T>(reinterpret_cast<const T *>(bias_bh)[o2]);
                     }
                 }
             }
-            // row statistics of this query block: staged in shared memory, else straight from global
-            const float *lse_blk = STAGE_STATS ? sm.lse_s[it & 1] : lse2_bh + blk0;
-            const float *dsc_blk = STAGE_STATS ? sm.dsc_s[it & 1] : ds_bh + blk0;
-            if (STAGE_STATS) {
+            // row statistics of this query block, staged in shared memory
+            const float *lse_blk = sm.lse_s[it & 1], *dsc_blk = sm.dsc_s[it & 1];
+            if (DKDV) {
                 ok = mbar_wait(&sm.y_full[it & 1], (uint32_t)(it >> 1) & 1u, status, 60);
                 if (!ok) break;
             }
@@ -390,55 +328,28 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_tmem(const __grid_con
                     tc_fence_before_sync();
                     mbar_arrive(&sm.p_ready);
                 }
-                if (!slow) {
-                    if (DKDV) {
-                        float4 l4[16];
+                tmem_wait_ld();
+                // Interior blocks with a bias need no mask either: rows past the end of Q have
+                // lse2 = +inf, which makes their P exactly 0 whatever the (clamped) bias holds.
+                const bool need_mask = diag || cta_key_tail || (!DKDV && blk0 + BT > p.Tk);
+                if (!need_mask) {
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) l4[i] = reinterpret_cast<const float4 *>(lse_blk + half * 64)[i];
-                        tmem_wait_ld();
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            pv[4 * i + 0] = ex2b(fmaf(__uint_as_float(ra[4 * i + 0]), p.scale_log2, -l4[i].x));
-                            pv[4 * i + 1] = ex2b(fmaf(__uint_as_float(ra[4 * i + 1]), p.scale_log2, -l4[i].y));
-                            pv[4 * i + 2] = ex2b(fmaf(__uint_as_float(ra[4 * i + 2]), p.scale_log2, -l4[i].z));
-                            pv[4 * i + 3] = ex2b(fmaf(__uint_as_float(ra[4 * i + 3]), p.scale_log2, -l4[i].w));
-                            pv[32 + 4 * i + 0] = ex2b(fmaf(__uint_as_float(rb[4 * i + 0]), p.scale_log2, -l4[8 + i].x));
-                            pv[32 + 4 * i + 1] = ex2b(fmaf(__uint_as_float(rb[4 * i + 1]), p.scale_log2, -l4[8 + i].y));
-                            pv[32 + 4 * i + 2] = ex2b(fmaf(__uint_as_float(rb[4 * i + 2]), p.scale_log2, -l4[8 + i].z));
-                            pv[32 + 4 * i + 3] = ex2b(fmaf(__uint_as_float(rb[4 * i + 3]), p.scale_log2, -l4[8 + i].w));
-                        }
-                    } else {
-                        tmem_wait_ld();
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) {
-                            pv[i] = ex2b(fmaf(__uint_as_float(ra[i]), p.scale_log2, -lse_row));
-                            pv[32 + i] = ex2b(fmaf(__uint_as_float(rb[i]), p.scale_log2, -lse_row));
-                        }
+                    for (int i = 0; i < 64; ++i) {
+                        float x = __uint_as_float(i < 32 ? ra[i & 31] : rb[i & 31]) * p.scale_log2;
+                        const float l2 = DKDV ? lse_blk[half * 64 + i] : lse_row;
+                        x = fmaf(bv[i], LOG2E, x);
+                        pv[i] = ex2b(x - l2);
                     }
                 } else {
-                    tmem_wait_ld();
-                    // Interior blocks with a bias need no mask either: rows past the end of Q have
-                    // lse2 = +inf, which makes their P exactly 0 whatever the (clamped) bias holds.
-                    const bool need_mask = diag || cta_key_tail || (!DKDV && blk0 + BT > p.Tk);
-                    if (!need_mask) {
 #pragma unroll
-                        for (int i = 0; i < 64; ++i) {
-                            float x = __uint_as_float(i < 32 ? ra[i & 31] : rb[i & 31]) * p.scale_log2;
-                            const float l2 = DKDV ? lse_blk[half * 64 + i] : lse_row;
-                            if constexpr (BIAS != 0) x = fmaf(bv[i], LOG2E, x);
-                            pv[i] = ex2b(x - l2);
-                        }
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 64; ++i) {
-                            const int col = c0 + i;
-                            const int qi = DKDV ? col : row, kj = DKDV ? row : col;
-                            float x = __uint_as_float(i < 32 ? ra[i & 31] : rb[i & 31]) * p.scale_log2;
-                            const bool masked = kj >= p.Tk || qi >= p.Tq || (p.causal && kj > qi);
-                            const float l2 = DKDV ? lse_blk[half * 64 + i] : lse_row;
-                            if constexpr (BIAS != 0) x = fmaf(bv[i], LOG2E, x);
-                            pv[i] = masked ? 0.f : ex2b(x - l2);
-                        }
+                    for (int i = 0; i < 64; ++i) {
+                        const int col = c0 + i;
+                        const int qi = DKDV ? col : row, kj = DKDV ? row : col;
+                        float x = __uint_as_float(i < 32 ? ra[i & 31] : rb[i & 31]) * p.scale_log2;
+                        const bool masked = kj >= p.Tk || qi >= p.Tq || (p.causal && kj > qi);
+                        const float l2 = DKDV ? lse_blk[half * 64 + i] : lse_row;
+                        x = fmaf(bv[i], LOG2E, x);
+                        pv[i] = masked ? 0.f : ex2b(x - l2);
                     }
                 }
                 if (DKDV) {
@@ -496,8 +407,6 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_tmem(const __grid_con
             }
             tc_fence_before_sync();
             mbar_arrive(&sm.ds_ready);
-            // dS, which depends on every bias value read above, has been stored: the bias stage is free
-            if constexpr (BIAS == 2) mbar_arrive(&sm.bb_empty[it % BSTAGES]);
         }
 
         // epilogue: accumulators -> global
@@ -641,7 +550,11 @@ __global__ void __launch_bounds__(DKDV_SUB_THREADS, 1) attn_bwd_dkdv_sub(const _
     tc_fence_after_sync();
     const uint32_t tbase = sm.tmem_base;
     grid_wait();            // the row statistics are in place
-    grid_trigger();         // the dQ kernel needs nothing from this one: it may fill the SMs this grid leaves idle
+    // The dQ kernel needs nothing from this one and may fill the SMs that this grid leaves idle.  It reads the row
+    // statistics without a wait of its own, which is sound because it starts only once EVERY CTA here has passed
+    // the wait above and this line: the trigger must stay behind the wait.  Its last CTA waits for this grid at its
+    // end, so whatever follows on the stream comes after both.
+    grid_trigger();
 
     if (warp == 8) {
         // ------------------------------ TMA producer ------------------------------
@@ -987,14 +900,14 @@ __global__ void __launch_bounds__(DKDV_SUB_THREADS, 1) attn_bwd_dkdv_sub(const _
 }
 
 // ---------------------------------------------------------------------------
-// Single-pass backward for head_dim 64: the dK/dV kernel above (same roles, tiles, tensor-memory
+// Single-pass backward for head dims up to 64: the dK/dV kernel above (same roles, tiles, tensor-memory
 // map and arithmetic: dK and dV are bit-identical to it) which ALSO forms the dQ partial tile of
 // every 128-query block, dQp = dS K, as a fifth GEMM from the dS^T it already holds, and adds it
 // to an fp32 accumulator in global memory with 16-byte vector reductions.  No second kernel
 // re-reads K, V (and the bias) or recomputes S, dP and the exponentials; a small kernel rounds
 // the accumulator into dQ afterwards.  As in the reference (tl.atomic_add into dq,
 // flash_attn_triton_cached.py:556-561) the order of the sums into dQ is not fixed: dQ may differ in
-// its last bits from run to run, dK and dV do not.  head_dim 64 leaves the 64 tensor-memory
+// its last bits from run to run, dK and dV do not.  64 channels leave the 64 tensor-memory
 // columns the partial tile needs (448..511) and the shared memory for dS^T (32 KB); at head_dim
 // 128 the same scheme is bound by the L2's reduction throughput and loses to the two-kernel form.
 // Four extra warps read the partial tiles back, so that reduction stalls do not hold up the
@@ -1015,17 +928,14 @@ struct alignas(1024) Single64Smem {
     uint64_t g1_free[2], g2_free[2];
     uint64_t bb_full[2], bb_empty[2];
     uint64_t dq_full, dq_read;                               // dQ partial tile complete / read back
-    int qblk[2];
     uint32_t tmem_base;
 };
 
 // BIASM: 0 no bias, 1 matrix bias staged by TMA, 2 vector bias.
 template <bool BF16, int BIASM>
 __global__ void __launch_bounds__(SINGLE64_THREADS, 1) attn_bwd_single64(const __grid_constant__ BwdTmaParams p) {
-    static_assert(BIASM >= 0 && BIASM <= 2, "no tile lists here");
     constexpr int D = 64;
     constexpr bool BIAS = BIASM == 1;
-    constexpr bool LISTS = false;
     using Smem = Single64Smem<BIAS>;
     constexpr bool STAGE_STATS = Smem::STAGE_STATS;
     constexpr uint32_t BIAS_BYTES = 64 * BT * 2;
@@ -1047,13 +957,7 @@ __global__ void __launch_bounds__(SINGLE64_THREADS, 1) attn_bwd_single64(const _
     const int r0 = blk * BT;                               // first key of this CTA
     const int i_begin = p.causal ? r0 / BT : 0;
     const int i_end = (p.Tq + BT - 1) / BT;
-    // With tile lists (matrix bias only) the CTA visits the listed query blocks: the count bounds
-    // every role's loop, the TMA producer alone reads the list and posts each stage's block index
-    // in shared memory (sm.qblk) before the stage's barrier, where the compute threads pick it up.
-    int tl_idx = -1;
-    if constexpr (LISTS)
-        tl_idx = (int)(((p.bias_b0 ? 0 : b) * (p.bias_h0 ? 1 : p.H) + (p.bias_h0 ? 0 : h)) * p.order.nblk + blk);
-    const int nit = LISTS ? (int)p.tlk_cnt[LISTS ? tl_idx : 0] : max(i_end - i_begin, 0);
+    const int nit = max(i_end - i_begin, 0);
     const int nsub = 2 * nit;
     int *status = p.status;
 
@@ -1104,20 +1008,12 @@ __global__ void __launch_bounds__(SINGLE64_THREADS, 1) attn_bwd_single64(const _
                 tma_load_4d(sm.x2 + hh * PANEL, &p.mv, &sm.x_full, hh * 64, r0, h, b);
             }
             bool ok = true;
-            // the list entry of the next block is fetched while waiting for this block's stage
-            const uint16_t *lst = LISTS ? p.tlk_list + (int64_t)tl_idx * p.tl_nqb : nullptr;
-            int qb_next = LISTS ? (int)lst[0] : 0;
             for (int it = 0; it < nit; ++it) {
                 const int s = it & 1;
                 const uint32_t ph = (uint32_t)(it >> 1) & 1u;
-                int qb = i_begin + it;
-                if constexpr (LISTS) {
-                    qb = qb_next;
-                    if (it + 1 < nit) qb_next = lst[it + 1];
-                }
+                const int qb = i_begin + it;
                 ok = mbar_wait(&sm.y_empty[s], ph ^ 1u, status, 71);
                 if (!ok) break;
-                if constexpr (LISTS) sm.qblk[s] = qb;   // ordered before the arrive below (release), read after the wait on y_full
                 mbar_expect_tx(&sm.y_full[s], 2 * TILE_BYTES + (STAGE_STATS ? 2 * BT * 4 : 0));
                 const int row = qb * BT;
                 if constexpr (STAGE_STATS) {
@@ -1305,13 +1201,7 @@ __global__ void __launch_bounds__(SINGLE64_THREADS, 1) attn_bwd_single64(const _
         for (int it = 0; it < nit; ++it) {
             const uint32_t par = (uint32_t)it & 1u;
             const int s = it & 1;
-            int blk0 = (i_begin + it) * BT;
-            if constexpr (LISTS) {
-                // the block's index is posted with its tiles
-                ok = mbar_wait(&sm.y_full[s], (uint32_t)(it >> 1) & 1u, status, 90);
-                if (!ok) break;
-                blk0 = sm.qblk[s] * BT;
-            }
+            const int blk0 = (i_begin + it) * BT;
             const int c0 = blk0 + sb * 64;                 // first query of the sub-block
             const bool slow = cta_key_tail || (p.causal && blk0 == r0);
             // row statistics of this sub-block's 64 queries: staged in shared memory, else from global
@@ -1321,11 +1211,9 @@ __global__ void __launch_bounds__(SINGLE64_THREADS, 1) attn_bwd_single64(const _
             const float4 *dsc4 = reinterpret_cast<const float4 *>(dsc_f);
             float pv[64];
 
-            if constexpr (!LISTS) {
-                // row statistics of this block have landed
-                ok = mbar_wait(&sm.y_full[s], (uint32_t)(it >> 1) & 1u, status, 90);
-                if (!ok) break;
-            }
+            // row statistics of this block have landed
+            ok = mbar_wait(&sm.y_full[s], (uint32_t)(it >> 1) & 1u, status, 90);
+            if (!ok) break;
 
             // x0[i] = bias * log2(e) - lse * log2(e) of query i (only -lse without a bias), formed
             // before the scores are waited for
@@ -2242,7 +2130,7 @@ __global__ void __launch_bounds__(DQ_PIPE_THREADS, 1) attn_bwd_dq_bias(const __g
 // scale, and lse * log2(e).  Rows in [Tq, Tq128) get +inf / 0 so that query
 // positions past the end need no masking in the main kernels.  One warp per row.
 // ---------------------------------------------------------------------------
-// Rounds the fp32 dQ accumulator of the single-pass backward ([B H][16][Tq128][4], head_dim 64) into
+// Rounds the fp32 dQ accumulator of the single-pass backward ([B H][16][Tq128][4], head_dim up to 64) into
 // dQ.  One CTA per 64 queries of one (batch, head): thread = (query, 16 channels).
 template <bool BF16>
 __global__ void __launch_bounds__(256) attn_bwd_dq_round64_kernel(const float *__restrict__ acc, void *dq, int64_t sb, int64_t sh,
@@ -2335,19 +2223,11 @@ bool tmem_bwd_eligible(const AttnParams &p) {
            heads_map_encodable(p.d_o, p.B, p.H, p.Tq, p.do_sb, p.do_sh, p.do_sn);
 }
 
-template <int D, bool BF16, bool DKDV, int BIAS>
-static int launch_bwd_one(const BwdTmaParams &bp, cudaStream_t st) {
-    constexpr int BSTAGES = BIAS == 2 ? (D == 64 ? 2 : 1) : 0;
-    const size_t smem = sizeof(BwdTmaSmem<D, BSTAGES>) + 1024;
-    if (int e = ensure_dyn_smem(reinterpret_cast<const void *>(attn_bwd_tmem<D, BF16, DKDV, BIAS>), smem)) return e;
-    return launch_pdl(attn_bwd_tmem<D, BF16, DKDV, BIAS>, bp.order.nblk * bp.order.BH, BWD_THREADS, smem, st, bp);
-}
-
 template <int D, bool BF16, bool DKDV>
 static int launch_bwd_tmem(const BwdTmaParams &bp, cudaStream_t st) {
-    if (bp.bias_kind != RGD_BIAS_NONE && bp.bias_vec == 2) return launch_bwd_one<D, BF16, DKDV, 2>(bp, st);
-    if (bp.bias_kind != RGD_BIAS_NONE) return launch_bwd_one<D, BF16, DKDV, 1>(bp, st);
-    return launch_bwd_one<D, BF16, DKDV, 0>(bp, st);
+    const size_t smem = sizeof(BwdTmaSmem<D>) + 1024;
+    if (int e = ensure_dyn_smem(reinterpret_cast<const void *>(attn_bwd_tmem<D, BF16, DKDV>), smem)) return e;
+    return launch_pdl(attn_bwd_tmem<D, BF16, DKDV>, bp.order.nblk * bp.order.BH, BWD_THREADS, smem, st, bp);
 }
 
 template <int D, bool BF16, int BIASM>
@@ -2357,8 +2237,9 @@ static int launch_dkdv_sub(const BwdTmaParams &bp, cudaStream_t st) {
     return launch_pdl(attn_bwd_dkdv_sub<D, BF16, BIASM>, bp.order.nblk * bp.order.BH, DKDV_SUB_THREADS, smem, st, bp);
 }
 
-// Single-pass form (head_dim 64): zero the accumulator, one kernel for dK, dV and the dQ partial sums,
-// round dQ.  bias_mode: 0 none, 1 matrix bias staged by TMA, 2 vector bias.
+// Single-pass form (head_dim up to 64): one kernel for dK, dV and the dQ partial sums, round dQ.  The accumulator
+// has been zeroed by attn_bwd_prep_kernel, which was launched with it.  bias_mode: 0 none, 1 matrix bias staged by
+// TMA, 2 vector bias.
 template <bool BF16>
 static int bwd_single64(const BwdTmaParams &bp, const AttnParams &p, int bias_mode, cudaStream_t st) {
     const size_t smem = (bias_mode == 1 ? sizeof(Single64Smem<true>) : sizeof(Single64Smem<false>)) + 1024;
