@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_tmem(const __grid_con
                 } else {
 #pragma unroll
                     for (int i = 0; i < 64; ++i) {
-                        const int64_t o2 = off + min(i, p.Tk - 1 - c0 < 0 ? 0 : p.Tk - 1 - c0);
+                        const int64_t o2 = off + min(i, p.Tk - 1 - c0);     // below 0 where the whole half lies past the keys
                         bv[i] = p.bias_f32 ? __ldg(reinterpret_cast<const float *>(bias_bh) + o2)
                                            : to_f32<T>(reinterpret_cast<const T *>(bias_bh)[o2]);
                     }

@@ -330,3 +330,13 @@ def test_nothing_is_written_past_the_channels(d, single, kind):
             assert torch.equal(a, b) or (single and i == 1 and (a - b).abs().max() <= 2.0 ** -8 * b.abs().max())
         for b, n in zip(bufs, (tq, tq, tk, tk)):
             assert (b[:8] == 7).all() and (b[-8:] == 7).all() and (b[8:-8].view(B, n, H, d + 8)[..., d:] == 7).all()
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("tk", [1, 40, 60, 65, 190, 193])
+def test_fp32_bias_with_half_a_block_past_the_keys(d, tk):
+    """A matrix bias that the threads read themselves: a block whose second 64 keys lie past the end reads nothing there
+    (the bias ends with its allocation's last row)."""
+    g = gen(tk)
+    q, k, v, do = _inputs(g, 2, 130, tk, 3, d, torch.bfloat16)
+    check(q, k, v, do, make_bias(g, "matrix_f32", 2, 3, 130, tk, torch.bfloat16), False, f"d={d} tk={tk}")
