@@ -75,8 +75,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int *s
 // Order in which a 1-D grid walks the (batch, head) x tile-block pairs.  Without a causal mask the
 // blocks of one head run next to each other (they share its K and V in L2).  Under a causal mask the
 // work per block differs, and the blocks of `group` heads are interleaved by rank, heaviest rank
-// first, so that the last CTAs to start are the lightest ones; the group is as many heads as L2
-// holds the operands of.
+// first, so that the last CTAs to start are the lightest ones.  A group has as many heads as 48 MB hold
+// the shared operands of, rounded so that all groups are about equal (a last group of a few heads is a
+// tail of its own).  Forward / forward + backward in us, measured in turns:
+//                            one head   12 MB       24 MB       48 MB       96 MB    48 MB, ragged last group
+//   [2, 3001, 16, 128]       117 / 453  101 / 418   97 / 416    97 / 417    97 / 417    97 / 417
+//   [2, 4608, 24, 64]        271 / 901  252 / 850   238 / 833   237 / 830   236 / 832   268 / 876
+//   [2, 2600, 20, 128]       121 / 456  113 / 434   110 / 431   103 / 424   100 / 424   123 / 465
+//   [2, 4096, 24, 128]       278 / 1138 261 / 1097  248 / 1088  247 / 1081  248 / 1099  242 / 1080
 // ---------------------------------------------------------------------------
 struct TileOrder {
     int nblk, group, BH;
@@ -89,8 +95,10 @@ __device__ __forceinline__ void tile_of(const TileOrder &o, int &rank, int &bh) 
     bh = g * o.group + rem - rank * heads;
 }
 inline TileOrder make_tile_order(int nblk, int BH, bool causal, int64_t bytes_per_head) {
+    if (!causal || BH <= 0) return {nblk, 1, BH};
     const int64_t fit = (48ll << 20) / (bytes_per_head > 0 ? bytes_per_head : 1);
-    return {nblk, causal ? (int)(fit < 1 ? 1 : fit > BH ? BH : fit) : 1, BH};
+    const int most = (int)(fit < 1 ? 1 : fit > BH ? BH : fit), groups = (BH - 1) / most + 1;
+    return {nblk, (BH - 1) / groups + 1, BH};
 }
 
 // Programmatic dependent launch: a kernel launched with launch_pdl may start while its predecessor in

@@ -278,9 +278,10 @@ def test_a_bias_is_not_scanned_on_its_first_call():
         assert torch.is_tensor(m.cache._tiles[2]) == (sight > 0)
 
 
-@pytest.mark.parametrize("d,H", [(128, 100), (64, 200)])
+@pytest.mark.parametrize("d,H", [(128, 101), (64, 201)])
 def test_causal_grid_of_more_heads_than_a_group_of_long_queries(d, H):
-    """As above for the dK/dV kernel, whose groups are sized by Q and dO: 95 / 190 heads of 1030 queries fit one."""
+    """As above for the dK/dV kernel, whose groups are sized by Q and dO: 95 / 190 heads of 1030 queries fit one.  Two
+    groups, one head apart in size."""
     g = gen(H + 1)
     q, k, v, do = (t.cuda() for t in _inputs(g, 1, 1030, 300, H, d, torch.bfloat16))
 
