@@ -261,11 +261,17 @@ template <typename T, int D>
 static int launch_few(const FewParams &fp, cudaStream_t st) {
     const AttnParams &p = fp.a;
     const int BH = p.B * p.H;
-    // Splits of a head's keys: as many CTAs as the chip holds at once (two per SM), at least one tile per
-    // warp.  More heads than that: quarters, so that the last CTAs to run leave little of the chip idle.
+    // Splits of a head's keys: as many CTAs as the chip holds at once (two per SM), at least one tile per warp.
+    // More heads than half of that fill the chip unsplit at head dims above 64, and below in halves (three CTAs share
+    // an SM there); quarters and eighths only add combining.  8 queries of 192 heads, us at 1 / 2 / 4 / 8 splits:
+    //   head_dim 128: 512 keys 14.9 / 18.7 / 24.9 / 45.5, 4096 keys 75.2 / 82.3 / 74.9 / 94.5
+    //   head_dim 64:  512 keys 12.6 / 10.9 / 16.8 / 32.8, 4096 keys 49.1 / 42.4 / 43.6 / 58.7
+    // and of 96 heads, head_dim 128: 512 keys 12.7 / 11.4 / 16.9 / 25.0, 4096 keys 47.6 / 41.5 / 48.7 / 51.5.
     const int room = 2 * num_sms();
+    const bool many = BH > room / 2;
     int split = 1;
-    while (split < FEW_CLUSTER && split * 2 * FEW_WARPS <= fp.ntiles && (BH > room / 2 ? split < 4 : split * 2 * BH <= room)) split *= 2;
+    while (split < (many ? (D > 64 ? 1 : 2) : FEW_CLUSTER) && split * 2 * FEW_WARPS <= fp.ntiles && (many || split * 2 * BH <= room))
+        split *= 2;
     const size_t smem = sizeof(FewSmem<T, D>);
     auto kernel = p.bias_kind == RGD_BIAS_NONE ? attn_few_kernel<T, D, false> : attn_few_kernel<T, D, true>;
     if (int e = ensure_dyn_smem(reinterpret_cast<const void *>(kernel), smem)) return e;

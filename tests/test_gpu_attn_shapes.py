@@ -341,3 +341,13 @@ def test_fp32_bias_with_half_a_block_past_the_keys(d, tk):
     g = gen(tk)
     q, k, v, do = _inputs(g, 2, 130, tk, 3, d, torch.bfloat16)
     check(q, k, v, do, make_bias(g, "matrix_f32", 2, 3, 130, tk, torch.bfloat16), False, f"d={d} tk={tk}")
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("H", [37, 75])
+def test_few_queries_around_the_heads_that_fill_the_chip(d, H):
+    """148 and 150 heads x sequences: the last that are split over a cluster by the room left, the first that are not."""
+    g = gen(H)
+    for tq, tk in [(1, 640), (16, 1030)]:
+        q, k, v, do = _inputs(g, 4 if H == 37 else 2, tq, tk, H, d, torch.bfloat16)
+        check(q, k, v, do, None, False, f"few H={H} d={d} ({tq},{tk})")
