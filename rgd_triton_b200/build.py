@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import argparse
 import concurrent.futures as cf
+import importlib.metadata
 import os
 import shutil
 import subprocess
@@ -24,6 +25,7 @@ OBJ = CSRC / "build"
 LIB = PKG / "librgd_b200.so"
 HOST_SRC = CSRC / "host" / "torch_host.cpp"
 HOST_LIB = PKG / "_host.so"
+HOST_STAMP = OBJ / "host_versions"       # the torch and Python that _host.so was built against
 INCLUDE = PKG.parent / "include"
 
 NVCC_FLAGS = [
@@ -67,7 +69,9 @@ def _compile(src: Path, force: bool, verbose: bool, ptxas_v: bool) -> tuple[Path
 def _build_host(force: bool, verbose: bool) -> None:
     """The extension module (plain C++ against torch's headers; it finds librgd_b200.so at run time)."""
     newest_dep = max(p.stat().st_mtime for p in (HOST_SRC, INCLUDE / "rgd_b200.h", Path(__file__)))
-    if not force and HOST_LIB.exists() and HOST_LIB.stat().st_mtime >= newest_dep:
+    versions = f"torch {importlib.metadata.version('torch')}, Python {sys.version}"
+    if not force and HOST_LIB.exists() and HOST_LIB.stat().st_mtime >= newest_dep and \
+            HOST_STAMP.exists() and HOST_STAMP.read_text() == versions:
         return
     import sysconfig
 
@@ -84,6 +88,7 @@ def _build_host(force: bool, verbose: bool) -> None:
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"g++ failed for {HOST_SRC.name}:\n{res.stdout}\n{res.stderr}")
+    HOST_STAMP.write_text(versions)
 
 
 def sources() -> list[Path]:

@@ -165,3 +165,27 @@ def test_launch_plans_belong_to_one_thread():
     t.start()
     t.join()
     assert theirs[0] is not mine and F_._plan(cache, "fwd", ("key",), lambda: None) is not theirs[0]
+
+
+def test_host_extension_is_rebuilt_for_another_torch(monkeypatch, tmp_path):
+    """_host.so uses torch's C++ classes: a build against another torch (or Python) does not count as current."""
+    from rgd_triton_b200 import build
+
+    build.build()
+    calls = []
+
+    def compiler(cmd, **kw):
+        calls.append(cmd)
+        return type("Result", (), {"returncode": 0, "stdout": "", "stderr": ""})
+    stamp = tmp_path / "versions"
+    stamp.write_text(build.HOST_STAMP.read_text())
+    monkeypatch.setattr(build, "HOST_STAMP", stamp)
+    monkeypatch.setattr(build.subprocess, "run", compiler)
+    build._build_host(False, False)
+    assert not calls
+    stamp.write_text("torch 1.0, Python 3.0")
+    build._build_host(False, False)
+    assert len(calls) == 1 and stamp.read_text() != "torch 1.0, Python 3.0"
+    stamp.unlink()
+    build._build_host(False, False)
+    assert len(calls) == 2
