@@ -22,7 +22,8 @@ Differences from the reference, all deliberate:
 * the entry points run on the native host path (``csrc/host/torch_host.cpp``: checks, allocation,
   launch and the autograd node in C++); what it does not cover comes back as None and is handled
   here, by the ``*_Func`` classes: arguments that are wrong (the exceptions are raised here), tensor
-  subclasses, channel strides other than 1, empty tensors, bias gradients, in-place rotation.
+  subclasses, channel strides other than 1, empty tensors, bias gradients, in-place rotation, calls
+  under a tracer, a dispatch mode or a functorch transform.
 * ``kernel_cache`` slots hold a validated launch key (shapes, strides, dtypes)
   instead of a compiled-kernel handle.  A call whose key differs re-validates
   and replaces the slot, so one module can be reused across shapes and dtypes
