@@ -698,6 +698,11 @@ bool addressable(const Tensor &t, bool zero_strides = false) {
 bool copies_pay(const Attn &a) {
     return a.d % 8 == 0 && a.d != 64 && a.d != 128 && a.B * a.H * a.tq * a.tk >= (int64_t)1 << 24;
 }
+// Outputs and gradients lie as the inputs do; those of the problems above are dense, as they were when these were
+// padded (a caller may view the heads and channels of a large output as one).
+Tensor attn_out(const Attn &a, const Tensor &t) {
+    return copies_pay(a) ? new_buffer(t.sizes(), t.scalar_type(), t.device()) : new_like(t);
+}
 
 struct AttnBackward : public Node {
     Attn a;
@@ -746,7 +751,7 @@ struct AttnBackward : public Node {
         if ((a.bias_sb == 0) == (this->a.bias_sb == 0) && (a.bias_sh == 0) == (this->a.bias_sh == 0)) tiles = this->tiles;
         Tensor dot = upstream(grads[0], qt);
         if (copies_pay(a) && !addressable(dot)) dot = dot.clone(at::MemoryFormat::Contiguous);
-        Tensor dq = new_like(qt), dk = new_like(kt), dv = new_like(vt);
+        Tensor dq = attn_out(a, qt), dk = attn_out(a, kt), dv = attn_out(a, vt);
         int64_t bytes = std::max<int64_t>(api.attn_bwd_workspace_bytes(a.B, a.H, a.tq, a.tk, a.d, a.dtype), 16);
         if (single_pass.load(std::memory_order_relaxed) && !tiles.defined())
             bytes = std::max(bytes, api.attn_bwd_single_pass_workspace_bytes(a.B, a.H, a.tq, a.tk, a.d, a.dtype));
@@ -768,7 +773,7 @@ PyObject *attn_call(Attn &a, const Tensor &q, const Tensor &k, const Tensor &v, 
     {
         NoGil nogil;
         c10::cuda::OptionalCUDAGuard guard(q.device());
-        o = new_like(q);
+        o = attn_out(a, q);
         lse = new_buffer({a.B, a.H, api.attn_lse_rows(a.tq)}, at::kFloat, q.device());
         const rgd_heads qv = Attn::view(q), kv = Attn::view(k), vv = Attn::view(v), ov = Attn::view(o);
         const rgd_bias b = a.bias(bias, tiles);

@@ -1036,7 +1036,8 @@ def flash_attn_func(q, k, v, bias=None, causal=False, softmax_scale=None, return
             return out
         if bias is not None and kernel_cache is not None:
             kernel_cache._tiles = seen          # what follows counts this call's sight of the bias itself
-    if d not in (0, 64, 128) and d % 8 == 0 and d < 128 and _pad_head_dim_pays(q, k):
+    large = d not in (0, 64, 128) and d % 8 == 0 and d < 128 and _pad_head_dim_pays(q, k)
+    if large:
         # Large problems of these head dims are worth a dense copy of what is not addressable (keys shared by the
         # heads, a slice at an odd offset; the native path hands them back): [2, 1100, 12, 96] with expanded keys
         # and values 114 us on the general kernels without the copy, 46 with it.  Head dims 64 and 128 keep to the
@@ -1049,4 +1050,6 @@ def flash_attn_func(q, k, v, bias=None, causal=False, softmax_scale=None, return
         _, _, _, o, lse, _, _, _ = _attn_forward(q, k, v, bias, causal, softmax_scale, kernel_cache)
     else:
         o, lse = FlashAttnFunc.apply(q, k, v, bias, causal, softmax_scale, kernel_cache)
+    if large:
+        o = o.contiguous()      # as the native path and the padded head dims return it
     return (o, lse) if return_lse else o

@@ -351,3 +351,24 @@ def test_few_queries_around_the_heads_that_fill_the_chip(d, H):
     for tq, tk in [(1, 640), (16, 1030)]:
         q, k, v, do = _inputs(g, 4 if H == 37 else 2, tq, tk, H, d, torch.bfloat16)
         check(q, k, v, do, None, False, f"few H={H} d={d} ({tq},{tk})")
+
+
+@pytest.mark.parametrize("native", [True, False])
+@pytest.mark.parametrize("d", [96, 100])
+def test_large_outputs_of_other_head_dims_are_dense(d, native, monkeypatch):
+    """Whatever the layout of q (heads second here): its heads and channels can be viewed as one dimension."""
+    if not native:
+        monkeypatch.setattr(F_, "_bind_host", lambda t: None)
+        monkeypatch.setattr(F_, "_HOST", None)
+    g = gen(d)
+    B, T, H = 2, 840, 12
+    heads_second = [randn(g, B, H, T, d, dtype=torch.bfloat16).cuda() for _ in range(3)]
+    q, k, v = (t.transpose(1, 2).requires_grad_(True) for t in heads_second)
+    o = F_.flash_attn_func(q, k, v)
+    assert o.view(B, T, H * d).shape == (B, T, H * d)
+    grads = torch.autograd.grad(o, (q, k, v), torch.ones_like(o))
+    assert [t.shape for t in grads] == [q.shape] * 3
+    if native:
+        assert all(t.is_contiguous() for t in grads)
+    dense = F_.flash_attn_func(*(t.transpose(1, 2).contiguous() for t in heads_second))
+    assert torch.equal(o, dense)
